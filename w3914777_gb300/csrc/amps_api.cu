@@ -39,10 +39,10 @@ struct amps_handle {
     void *store[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     int parity = 0;
     bool transition = false;  // next step reads tiles at tier_prev
-    // every tile is at FP64 until the next classification (the first period
-    // of a temporal / rate monitor): grain growth takes the staged FP64 kernel
-    // when it is prepared (stage64: its FP64 staging fits in shared memory)
-    bool all_fp64 = false, stage64 = false;
+    // grain growth: every tile is at FP64 until the next classification (the
+    // first period of a temporal / rate monitor), so the steps fetch no FP32
+    // neighbourhoods speculatively
+    bool all_fp64 = false;
     uint8_t *d_tier_prev = nullptr, *d_tier_cur = nullptr;
     int *d_lists = nullptr, *d_counts = nullptr;
     int *d_order = nullptr;  // launch order of the fused grain-growth step (adaptive runs)
@@ -167,6 +167,17 @@ static bool encode_field_map(CUtensorMap *tm, void *base, int nx, int ny, int nf
 
 static size_t tier_size(int t) { return t == TIER_FP64 ? 8 : (t == TIER_FP32 ? 4 : 2); }
 
+// How div_known divides by d.
+static int div_kind(double d)
+{
+    int ex;
+    const double m = std::fabs(std::frexp(d, &ex));
+    if (!(m >= 0.5) || ex < -63 || ex > 64) return DIV_GENERAL;
+    if (m == 0.5) return DIV_MUL;
+    // the relative error of RN(1/d), exact through the fused multiply-add
+    return std::fabs(std::fma(-d, 1.0 / d, 1.0)) <= std::ldexp(1.0, -54) ? DIV_KNOWN : DIV_GENERAL;
+}
+
 static Phys make_phys(const amps_params &p)
 {
     Phys ph;
@@ -174,6 +185,7 @@ static Phys make_phys(const amps_params &p)
     ph.dx = p.dx; ph.dy = p.dy; ph.dt = p.dt;
     ph.dxdy = p.dx * p.dy;
     ph.inv_dxdy = 1.0 / ph.dxdy;
+    ph.dxdy_div = div_kind(ph.dxdy);
     ph.tau = p.tau; ph.epsb = p.epsb; ph.kappa = p.kappa; ph.delta = p.delta; ph.aniso = p.aniso;
     ph.alpha = p.alpha; ph.gama = p.gama; ph.teq = p.teq; ph.theta0 = p.theta0; ph.pi = p.pi; ph.noise = p.noise;
     ph.mobil = p.mobil; ph.grcoef = p.grcoef; ph.gamma = p.gamma;
@@ -201,6 +213,9 @@ static Phys make_phys(const amps_params &p)
         const bool even = ph.aniso >= 2 && ph.aniso <= 16 && ph.aniso == 2 * std::floor(ph.aniso / 2);
         k[KB_MODE] = even ? ph.aniso : 0;
         k[KB_C0] = std::cos(ph.aniso * ph.theta0); k[KB_S0] = std::sin(ph.aniso * ph.theta0);
+    } else if (p.model == AMPS_GRAINGROWTH) {
+        k[GG_G2] = 2.0 * ph.gamma; k[GG_M2] = 1.0 - 2.0 * ph.gamma; k[GG_KI] = ph.grcoef * ph.inv_dxdy;
+        k[GG_DTM] = ph.dt * ph.mobil;
     } else if (p.model == AMPS_SINTERING) {
         k[SN_INV] = ph.inv_dxdy; k[SN_B] = ph.B; k[SN_A2] = 2.0 * ph.A; k[SN_HCM] = 0.5 * ph.coefm;
         k[SN_DVOL] = ph.dvol; k[SN_DVAP] = ph.dvap; k[SN_DSUR] = ph.dsur; k[SN_DGRB] = ph.dgrb; k[SN_DT] = ph.dt;
@@ -212,7 +227,12 @@ static Phys make_phys(const amps_params &p)
 
 static size_t kernel_smem(const amps_params &p, int tier, int nf, bool only64)
 {
-    if (p.model == AMPS_GRAINGROWTH) return gg_smem_bytes(p.tile, only64 ? TIER_FP64 : -1, nf);
+    if (p.model == AMPS_GRAINGROWTH) {
+        // a plain FP64 run is held to its whole tile's FP64 neighbourhood, as ever
+        // (its steps stage less: bands of rows)
+        if (only64) return (size_t)nf * (p.tile == 32 ? Stage<double, 32, 1>::FIELD : Stage<double, 16, 1>::FIELD) * 8;
+        return gg_smem_bytes(p.tile, nf);
+    }
     if (p.model == AMPS_KOBAYASHI) return kob_smem_bytes(p.tile, tier);
     return sint_smem_bytes(p.tile, tier, nf, p.mu_lap_fp64 || tier == TIER_FP64);
 }
@@ -330,10 +350,7 @@ extern "C" int amps_create(const amps_params *p, amps_handle **out)
     for (int t = 0; t < 3; ++t) {
         if (!h->used[t]) continue;
         cudaError_t pe;
-        if (p->model == AMPS_GRAINGROWTH) {
-            const bool only64 = h->used[TIER_FP64] && !h->used[TIER_FP32] && !h->used[TIER_HALF];
-            pe = gg_prepare(h->T, only64 ? TIER_FP64 : -1, p->ref_order != 0, p->half_arith, h->ragged);
-        }
+        if (p->model == AMPS_GRAINGROWTH) pe = gg_prepare(h->T, p->ref_order != 0, p->half_arith, h->ragged);
         else if (p->model == AMPS_KOBAYASHI) pe = kob_prepare(h->T, t, p->ref_order != 0);
         else pe = sint_prepare(h->T, t, p->ref_order != 0, p->mu_lap_fp64 != 0);
         if (pe == cudaSuccess && p->model != AMPS_GRAINGROWTH && t == TIER_FP32 && h->used[TIER_HALF])
@@ -345,11 +362,6 @@ extern "C" int amps_create(const amps_params *p, amps_handle **out)
             return AMPS_ERR_CUDA;
         }
     }
-    // adaptive grain growth with an FP64 high tier: the staged FP64 kernel for
-    // periods whose tiles are all FP64 (a refused attribute leaves the fused kernel)
-    if (p->model == AMPS_GRAINGROWTH && h->mixed && high == TIER_FP64 &&
-        kernel_smem(*p, TIER_FP64, h->nf, true) <= (size_t)kMaxDynSmem)
-        h->stage64 = gg_prepare(h->T, TIER_FP64, p->ref_order != 0, 0) == cudaSuccess;
     cudaGetLastError();
     {
         // grain growth, 32x32 tiles, an FP32 tier: tensor maps of the two FP32
@@ -474,7 +486,7 @@ static int reclassify_resting(amps_handle *h)
                 CK(h, monitor_state(g, 2, p.monitor_samples, p.monitor_field, nullptr, h->d_snap, 1, h->d_flags,
                                     h->stream));
             // every tile to the high tier for the first period
-            h->all_fp64 = h->stage64 && h->sched_n == 0;
+            h->all_fp64 = p.model == AMPS_GRAINGROWTH && p.high_tier == TIER_FP64 && h->sched_n == 0 && p.thr_hi <= 1e300;
             std::vector<double> big(h->ntiles, 1e300);
             CK(h, cudaMemcpyAsync(h->d_metric, big.data(), sizeof(double) * h->ntiles, cudaMemcpyHostToDevice, h->stream));
             CK(h, cudaStreamSynchronize(h->stream));
@@ -626,7 +638,8 @@ extern "C" int amps_get_fields(amps_handle *h, void *dst, int dtype, int on_devi
 // -------------------------------------------------------------- time loop ----
 // Arguments of the step at offset step_off of a period, from parity
 // `parity` (transition: this step reads tiles at their previous tier).
-static StepArgs step_args(const amps_handle *h, int parity, bool transition, int step_off, bool monitor_now)
+static StepArgs step_args(const amps_handle *h, int parity, bool transition, int step_off, bool monitor_now,
+                          bool all64 = false)
 {
     const amps_params &p = h->p;
     StepArgs a;
@@ -650,6 +663,7 @@ static StepArgs step_args(const amps_handle *h, int parity, bool transition, int
     a.mu_lap_fp64 = p.mu_lap_fp64;
     a.cadence = p.cadence;
     a.half_arith = p.half_arith;
+    a.all64 = all64 ? 1 : 0;
     a.tma_stage = h->tma_stage ? 1 : 0;
     a.metric = h->d_metric;
     a.snap = h->d_snap;
@@ -690,15 +704,12 @@ static int prof_begin(amps_handle *h, amps_handle::Ev &ev)
 static int launch_step(amps_handle *h, int step_off, bool monitor_now)
 {
     const amps_params &p = h->p;
-    StepArgs a = step_args(h, h->parity, h->transition, step_off, monitor_now);
+    StepArgs a = step_args(h, h->parity, h->transition, step_off, monitor_now, h->all_fp64);
     const bool ref = p.ref_order != 0;
     if (p.model == AMPS_GRAINGROWTH) {
         // one fused launch covers every tier (profiled per chunk by enqueue_chunk)
-        // all-FP64 runs and steps use the staged FP64 kernel, every other the fused one
-        const bool only64 = (h->used[TIER_FP64] && !h->used[TIER_FP32] && !h->used[TIER_HALF]) ||
-                            (h->all_fp64 && !monitor_now);
         cudaError_t e = h->use_tma ? gg_launch_tma(ref, h->tm[h->parity], a, h->tma_grid, h->stream)
-                                   : gg_launch(h->T, only64 ? TIER_FP64 : -1, ref, a, h->ntiles, h->stream,
+                                   : gg_launch(h->T, ref, a, h->ntiles, h->stream,
                                                h->tma_stage ? &h->tm[h->parity] : nullptr);
         if (e != cudaSuccess) FAIL(h, AMPS_ERR_CUDA, "step kernel launch: %s", cudaGetErrorString(e));
         ++h->launches;
@@ -1478,7 +1489,7 @@ static std::vector<StepArgs> ens_tables(const amps_ensemble *e, int k0, int cnt)
         bool tr = h->transition;
         for (int s = 0; s < cnt; ++s) {
             const bool mon = e->mixed && period_end && s == cnt - 1;
-            t[(size_t)s * M + i] = step_args(h, par, tr, k0 + s, mon);
+            t[(size_t)s * M + i] = step_args(h, par, tr, k0 + s, mon, h->all_fp64);
             if (e->d_tmaps && h->tma_stage) {
                 t[(size_t)s * M + i].tmap = e->d_tmaps + 4 * i + par;
                 // split-tile boxes where they were encoded (else per-thread copies)
@@ -1558,7 +1569,7 @@ extern "C" int amps_ensemble_run(amps_ensemble *e, int nsteps)
         const bool period_end = k0 + cnt == e->cad;
         if (e->graphs && k0 == 0 && cnt == e->cad) {
             std::vector<uint8_t> key(M);
-            for (int i = 0; i < M; ++i) key[i] = (uint8_t)(e->m[i]->parity | (e->m[i]->transition ? 2 : 0));
+            for (int i = 0; i < M; ++i) key[i] = (uint8_t)(e->m[i]->parity | (e->m[i]->transition ? 2 : 0) | (e->m[i]->all_fp64 ? 4 : 0));
             auto it = e->periods.find(key);
             if (it == e->periods.end()) {
                 const std::vector<StepArgs> tab = ens_tables(e, 0, cnt);

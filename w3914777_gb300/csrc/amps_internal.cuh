@@ -25,6 +25,7 @@ enum { TIER_HALF = 0, TIER_FP32 = 1, TIER_FP64 = 2 };
 // Model constants (double; each kernel rounds them to its compute type).
 struct Phys {
     double dx, dy, dt, dxdy, inv_dxdy;
+    int dxdy_div;  // how div_known divides by dx*dy (enum DivKind)
     // Kobayashi
     double tau, epsb, kappa, delta, aniso, alpha, gama, teq, theta0, pi, noise;
     // grain growth
@@ -60,6 +61,8 @@ enum KConst {
     KB_KAPPA, KB_DT, KB_INV, KB_MODE, KB_C0, KB_S0,
     // sintering: 1/dxdy, B, 2A, 0.5*coefm, dvol, dvap, dsur, dgrb, dt, 12B, dt*coefl, 0.5*coefk
     SN_INV = 0, SN_B, SN_A2, SN_HCM, SN_DVOL, SN_DVAP, SN_DSUR, SN_DGRB, SN_DT, SN_B12, SN_DTL, SN_HCK,
+    // grain growth's FP64 tiles: 2*gamma, 1 - 2*gamma, kappa/(dx*dy), dt*L
+    GG_G2 = 0, GG_M2, GG_KI, GG_DTM,
     KCONST_MAX = 24
 };
 
@@ -89,6 +92,7 @@ struct StepArgs {
     // monitor (active when monitor_now != 0)
     int monitor_now, monitor_kind, samples, mfield, mu_lap_fp64, cadence;
     int half_arith;           // grain growth: AMPS_HALF_FP32 / _REF / _HFMA2 (half tiles' arithmetic)
+    int all64;                // grain growth: every tile of this step is read and written at FP64
     int tma_stage;            // grain growth: the launch carries a tensor map of the FP32 input (bulk staging)
     const CUtensorMap *tmap;  // ensemble steps: the member's tensor map of its FP32 input in global memory (or null)
     const CUtensorMap *tmap8; // ensemble split tiles: the same input with boxes of kPairFields fields (or null)
@@ -208,7 +212,27 @@ __device__ __forceinline__ double cube_rn(double x)
 {
     const double p = __dmul_rn(x, x), pe = __fma_rn(x, x, -p);
     const double hi = __dmul_rn(p, x), he = __fma_rn(p, x, -hi);
-    return __dadd_rn(hi, __dadd_rn(he, __dmul_rn(pe, x)));
+    const double r = __dadd_rn(hi, __dadd_rn(he, __dmul_rn(pe, x)));
+    return (__double2hiint(hi) & 0x7ff00000) == 0x7ff00000 ? hi : r;  // infinite: he would be NaN
+}
+
+// x / d rounded to nearest (IEEE) for a divisor known in advance; inv = RN(1/d).
+// DIV_MUL (d a power of two): the product is the quotient.  DIV_KNOWN (the host
+// found inv within 2^-54 of 1/d, relatively): q = x*inv is then within an ulp of
+// x/d, its remainder is exact, and Markstein's correction ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990) gives the
+// rounded quotient -- 3 FP64 operations against ~10 and a branch of the general
+// division.  Zero keeps its sign; tiny, huge, infinite and NaN x, whose
+// remainders need not be exact, take the general division, as does every x of
+// any other divisor (DIV_GENERAL).
+enum DivKind { DIV_GENERAL, DIV_MUL, DIV_KNOWN };
+__device__ __forceinline__ double div_known(double x, double d, double inv, int kind)
+{
+    if (kind == DIV_GENERAL) return __ddiv_rn(x, d);
+    const double q = __dmul_rn(x, inv);
+    if (kind == DIV_MUL || pos_zero(fabs(x))) return q;
+    if ((unsigned)((__double2hiint(x) >> 20 & 0x7ff) - 128) > 1792u) return __ddiv_rn(x, d);
+    return __fma_rn(__fma_rn(-q, d, x), inv, q);
 }
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

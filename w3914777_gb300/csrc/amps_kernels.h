@@ -5,13 +5,13 @@
 namespace amps {
 
 // tm (nullable): tensor map of the step's FP32 input, used when a.tma_stage.
-cudaError_t gg_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s,
+cudaError_t gg_launch(int tile, bool ref, const StepArgs &a, int grid, cudaStream_t s,
                       const CUtensorMap *tm = nullptr);
 // pdl: launched programmatically after the stream's previous grid (the kernel waits for it first)
 cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl = false);
 cudaError_t sint_launch(int tile, int tier, bool ref, bool mu64, const StepArgs &a, int grid, cudaStream_t s,
                         bool pdl = false);
-size_t gg_smem_bytes(int tile, int tier, int nf);
+size_t gg_smem_bytes(int tile, int nf);
 // Kobayashi / sintering: the half and FP32 tiles of a step in one launch
 // (grid = all tiles; FP64 tiles are skipped, left to the FP64 tier launch).
 // after64: this step's FP64 launch directly precedes (run alongside it)
@@ -22,7 +22,7 @@ cudaError_t sint_prepare_lo(int tile, bool mu64);
 // Raise the dynamic shared-memory limit of the kernel a launch would use
 // (must run before any graph capture).
 // ragged: a side is not a multiple of the tile (the partial-edge-tile kernels).
-cudaError_t gg_prepare(int tile, int tier, bool ref, int half_arith, bool ragged = false);
+cudaError_t gg_prepare(int tile, bool ref, int half_arith, bool ragged = false);
 // The fused step with binary16 arithmetic on half tiles (half_arith 1 or 2;
 // k_gg_half.cu), called by gg_launch / gg_prepare.
 cudaError_t gg_launch_half(int tile, bool ref, const StepArgs &a, int grid, size_t smem, cudaStream_t s,

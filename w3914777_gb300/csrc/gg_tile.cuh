@@ -219,120 +219,286 @@ __device__ __forceinline__ void gg_tile_lo_rows(const StepArgs &a, const float *
     }
 }
 
-// One cell of the FP64 tile's neighbourhood at tile-local (ly, lx), read at
+// ---- FP64 tiles --------------------------------------------------------------
+// Bound by the FP64 pipe (1.25 TFLOP/s nominal, ~1/60 of FP32): everything
+// here is arranged for few FP64 operations a cell and field, and the rest
+// (staging, shared-memory traffic, index arithmetic) hides behind them.
+//
+// A tile is advanced in bands of HB rows: the band's rows and a 1-cell halo of
+// every field are staged as doubles in the memory the FP32 tiles stage in
+// (half the rows at twice the size: gg_fp64_band), then a lane sweeps RR rows
+// x 2 columns of one field.
+//
+// Library order (REF = false).  With the 3x3 box sum B (eight neighbours plus
+// the cell), S = sum_j eta_j^2 and G = 2 gamma S - 1, the update is
+//   eta' = eta - dtL*(eta*(G + (1 - 2 gamma) eta^2) - kappa/dxdy*(B - 9 eta)).
+// G is formed once per cell for all fields (into shared memory).  B shares its
+// partial sums: the middle pair of the two columns' row sums, and the middle
+// pair of rows of two output rows: 10.4 FP64 operations a cell and field
+// (eight rows a lane) in place of the 18 of eight separate neighbours.  9 eta
+// is taken off the pair of rows before the third is added: partial sums stay
+// below 6 eta and the last addition is of opposite numbers, so the error
+// against extended precision is that of the eight-neighbour form (equal to a
+// few percent over 200 steps of a polycrystal).
+// Which additions pair up depends on the parity of the tile-local row and
+// column, so every launch that computes a cell gets the same bits.
+// 5-point stencil: (left + right) + (up + down) - 4 eta.
+//
+// REF: the reference's expression order, every operation rounded on its own
+// (graingrowth/function.h:20-23); 8*eta is exact, so its subtraction is one
+// fused operation; the division by dx*dy is div_known; pow(eta, 3) is the
+// correctly rounded cube (cube_rn), within an ulp of any library's pow.  About
+// 27 FP64 operations a cell and field at Q = 2 in place of ~137 with pow and
+// the general division: 32 us a step in place of 103 on the reference's 512^2
+// two-field adaptive run, nearly all of whose 16^2 tiles hold a moving boundary.
+template <int T> struct Stage64 {
+    static constexpr int O = 2, P = T + 2 * O;  // interior at column 2: 16-byte aligned rows
+    __host__ __device__ static constexpr int field(int hb) { return (hb + 2) * P; }
+};
+
+// Rows of a band of `nf` fields: the most that fit in the FP32 staging of a
+// 32^2 tile (16 rows of 36 doubles against 34 of 40 floats, and the sum tile
+// in that of the sums of squares); a 16^2 tile whole, up to 16 fields.
+__host__ __device__ __forceinline__ int gg_fp64_band(int tile, int nf) { return tile == 32 ? 16 : (nf <= 16 ? 16 : 8); }
+
+// Stage rows [r0 - 1, r0 + hb] of every field (tile-local), each cell read at
 // its owner tile's input tier: the tile of the 3x3 neighbourhood at that
 // position, or (own: a ragged grid's edge tile, whose boundary-mapped halo
-// can lie in another tile) the tile that holds the mapped cell.
-template <int T>
-__device__ __forceinline__ double ld_nb64(const StepArgs &a, const uint8_t *nt, int f, int x0, int y0, int ly, int lx,
-                                          bool own = false)
+// can lie in another tile) the tile that holds the mapped cell.  FP64 cells by
+// asynchronous copies, every field in flight at once.
+// ALL64: every cell is at FP64 (no tier is looked up).
+template <int T, bool NC, bool ALL64 = false>
+__device__ __forceinline__ void gg_stage64(const StepArgs &a, double *sm, const uint8_t *nt, int x0, int y0, int r0,
+                                           int hb, bool own)
 {
-    const int gy = bc_map(y0 + ly, a.ny, a.bc), gx = bc_map(x0 + lx, a.nx, a.bc);
-    const int cls = (ly < 0 ? 0 : (ly < T ? 3 : 6)) + (lx < 0 ? 0 : (lx < T ? 1 : 2));
-    const int tier = own ? a.tier_in[(gy / T) * a.ntx + gx / T] : nt[cls];
-    return load_tier<double>(a, tier, (int64_t)f * a.n + (int64_t)gy * a.px + gx);
+    using S = Stage64<T>;
+    const int nf = a.nf, fs = S::field(hb);
+    for (int u = threadIdx.x; u < (hb + 2) * (T + 2); u += kThreads) {
+        const int ly = r0 - 1 + u / (T + 2), lx = u % (T + 2) - 1;
+        const int gy = bc_map(y0 + ly, a.ny, a.bc), gx = bc_map(x0 + lx, a.nx, a.bc);
+        const int cls = (ly < 0 ? 0 : (ly < T ? 3 : 6)) + (lx < 0 ? 0 : (lx < T ? 1 : 2));
+        const int tier = ALL64 ? TIER_FP64 : own ? a.tier_in[(gy / T) * a.ntx + gx / T] : nt[cls];
+        const int64_t g = (int64_t)gy * a.px + gx;
+        double *d = sm + (ly - r0 + 1) * S::P + S::O + lx;
+        if (NC && tier == TIER_FP64) {
+            const double *src = (const double *)a.in[TIER_FP64] + g;
+            for (int f = 0; f < nf; ++f)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d + f * fs)),
+                             "l"(src + (int64_t)f * a.n)
+                             : "memory");
+        } else {
+#pragma unroll 4
+            for (int f = 0; f < nf; ++f) {
+                const int64_t k = (int64_t)f * a.n + g;
+                if (tier == TIER_FP64) d[f * fs] = __ldcg((const double *)a.in[TIER_FP64] + k);
+                else if (tier == TIER_FP32) d[f * fs] = (double)ldro<NC>((const float *)a.in[TIER_FP32] + k);
+                else d[f * fs] = (double)__half2float(__ushort_as_half(ldro<NC>((const unsigned short *)a.in[TIER_HALF] + k)));
+            }
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_async_wait_all();
 }
 
-// FP64 tile: direct loads through L1 with a rolling 3-row window, FP64
-// arithmetic; REF keeps the reference's expression order and rounding
-// (graingrowth/function.h:20-23).
-// PH > 0: this CTA updates fields [f0, f0 + PH) of the tile (one CTA of a
-// split tile; the sum of squares still covers every field).
-template <int T, bool REF, bool PARTIAL = false, int PH = 0>
-__device__ __forceinline__ void gg_tile_fp64(const StepArgs &a, const uint8_t *nt, int tile, int tx, int ty, double *red,
-                                             int f0 = 0)
+// The monitor of an FP64 tile, from the values just stored (exact) and the
+// tile's input: one pass over the tile after the update, on monitor steps only.
+template <int T, int KIND>
+__device__ __forceinline__ void gg_monitor64(const StepArgs &a, const uint8_t *nt, int tile, int tx, int ty, double *red)
 {
-    constexpr bool partial = PARTIAL;  // a ragged grid's edge tile: owner-tier loads
-    constexpr int RPT = T * T / kThreads;
-    const int col = threadIdx.x % T;
-    const int r0 = (threadIdx.x / T) * RPT;
     const int x0 = tx * T, y0 = ty * T;
-    const int nf = a.nf;
-    const Phys &ph = a.ph;
-    double ssum[RPT];
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) ssum[j] = 0.0;
-    if (!REF)
-        for (int f = 0; f < nf; ++f)
-#pragma unroll
-            for (int j = 0; j < RPT; ++j) {
-                const double v = ld_nb64<T>(a, nt, f, x0, y0, r0 + j, col, partial);
-                ssum[j] = fma(v, v, ssum[j]);
-            }
-    const int64_t gbase = (int64_t)(y0 + r0) * a.px + x0 + col;
+    // a ragged grid's edge tile: cells past the domain are not samples
+    const int vw = min(T, a.nx - x0), vh = min(T, a.ny - y0);
+    constexpr bool range = KIND == 1;  // one reduction per field; the other kinds are maxima over fields
     double metric = 0.0;
     MonAcc mon;
-    for (int f = PH ? f0 : 0; f < (PH ? f0 + PH : nf); ++f) {
-        const bool mon_f = a.monitor_now && (a.mfield < 0 || a.mfield == f);
+    mon_reset(a, mon);
+    for (int f = 0; f < a.nf; ++f) {
+        if (a.mfield >= 0 && a.mfield != f) continue;
         const int mslot = a.mfield < 0 ? f : 0;
-        if (mon_f) mon_reset(a, mon);
-        double rd[3], rc[3], ru[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            rd[k] = ld_nb64<T>(a, nt, f, x0, y0, r0 - 1, col + k - 1, partial);
-            rc[k] = ld_nb64<T>(a, nt, f, x0, y0, r0, col + k - 1, partial);
-        }
-#pragma unroll 1
-        for (int j = 0; j < RPT; ++j) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) ru[k] = ld_nb64<T>(a, nt, f, x0, y0, r0 + j + 1, col + k - 1, partial);
-            const int64_t g = gbase + (int64_t)j * a.px;
-            const double snapv = mon_f ? snap_prefetch<T>(a, mslot, tile, r0 + j, col, g) : 0.0;
-            const double e = rc[1];
-            double out;
-            if (REF) {
-                double lap;
-                if (a.stencil == 0)
-                    lap = __ddiv_rn(__dsub_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(
-                                      rd[0], rd[1]), rd[2]), rc[0]), rc[2]), ru[0]), ru[1]), ru[2]),
-                                      __dmul_rn(8.0, e)), ph.dxdy);
-                else
-                    lap = __ddiv_rn(__dsub_rn(__dadd_rn(__dadd_rn(__dadd_rn(rc[0], rc[2]), rd[1]), ru[1]),
-                                              __dmul_rn(4.0, e)), ph.dxdy);
-                double sum = 0.0;
-                bool first = true;
-                for (int b = 0; b < nf; ++b) {
-                    if (b == f) continue;
-                    const double v = ld_nb64<T>(a, nt, b, x0, y0, r0 + j, col, partial);
-                    const double s2 = __dmul_rn(v, v);
-                    sum = first ? s2 : __dadd_rn(sum, s2);
-                    first = false;
-                }
-                const double dfd = __dsub_rn(__dadd_rn(__dmul_rn(__dmul_rn(2.0 * ph.gamma, e), sum), pow(e, 3.0)), e);
-                out = __dsub_rn(e, __dmul_rn(ph.dt * ph.mobil, __dsub_rn(dfd, __dmul_rn(ph.grcoef, lap))));
+        if (range) mon_reset(a, mon);
+        for (int u = threadIdx.x; u < T * T; u += kThreads) {
+            const int row = u / T, col = u % T;
+            if (row >= vh || col >= vw) continue;
+            const int64_t g = (int64_t)(y0 + row) * a.px + x0 + col, k = (int64_t)f * a.n + g;
+            const double v = ((const double *)a.out[TIER_FP64])[k];
+            if constexpr (KIND == 3) {
+                if ((__double2hiint(v) & 0x7ff00000) == 0x7ff00000) mon.bad = 1;
+                if (sample_index<T>(2, a.samples, row, col) >= 0)
+                    mon.dmaxf = fmaxf(mon.dmaxf, fabsf((float)v - load_tier<float>(a, nt[4], k)));
             } else {
-                double s;
-                if (a.stencil == 0) s = (rd[0] + rd[1] + rd[2]) + (rc[0] + rc[2]) + (ru[0] + ru[1] + ru[2]) - 8.0 * e;
-                else s = (rc[0] + rc[2]) + (rd[1] + ru[1]) - 4.0 * e;
-                const double lap = s * ph.inv_dxdy;
-                const double e2 = e * e;
-                double sj = ssum[0];
-#pragma unroll
-                for (int q = 1; q < RPT; ++q) sj = j == q ? ssum[q] : sj;
-                const double dfd = e * fma(2.0 * ph.gamma, sj - e2, e2 - 1.0);
-                out = fma(-(ph.dt * ph.mobil), fma(-ph.grcoef, lap, dfd), e);
-            }
-            ((double *)a.out[TIER_FP64])[(int64_t)f * a.n + g] = out;
-            // a ragged grid's edge tile: cells past the domain are not samples
-            if (mon_f && (!PARTIAL || (r0 + j < a.ny - y0 && col < a.nx - x0)))
-                mon_add<T>(a, mon, mslot, tile, r0 + j, col, g, out, e, snapv);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                rd[k] = rc[k];
-                rc[k] = ru[k];
+                mon_add<T>(a, mon, mslot, tile, row, col, g, v, 0.0, snap_prefetch<T>(a, mslot, tile, row, col, g));
             }
         }
-        if (mon_f) metric = mon_finish(a, mon, red, metric);
+        if (range) metric = mon_finish(a, mon, red, metric);
     }
-    if (a.monitor_now && threadIdx.x == 0) a.metric[tile] = metric;
+    if (!range) metric = mon_finish(a, mon, red, metric);
+    if (threadIdx.x == 0) a.metric[tile] = metric;
 }
 
-// The FP64 tile of a ragged grid's edge, out of line (off the whole tiles' registers).
-template <int T, bool REF, int PH = 0>
-__device__ __noinline__ void gg_tile_fp64_partial(const StepArgs &a, const uint8_t *nt, int tile, int tx, int ty,
-                                                  double *red, int f0 = 0)
+// The update of one band from its staging (rows [r0, r0 + hb) of the tile),
+// fields [f0, f0 + fn) (the sums cover every field).
+template <int T, bool REF, int RR>
+__device__ __forceinline__ void gg_band64(const StepArgs &a, const double *sm, double *ss, int x0, int y0, int r0,
+                                          int hb, int rot)
 {
-    gg_tile_fp64<T, REF, true, PH>(a, nt, tile, tx, ty, red, f0);
+    using S = Stage64<T>;
+    constexpr int GPR = T / 2, RG = 32 / GPR;  // column pairs a row, row groups a warp
+    const int nf = a.nf, fs = S::field(hb);
+    const Phys &ph = a.ph;
+    if (!REF) {
+        // G = 2 gamma S - 1 at every cell of the band
+        for (int u = threadIdx.x; u < hb * GPR; u += kThreads) {
+            const int row = u / GPR, c = 2 * (u % GPR);
+            const double *p = sm + (row + 1) * S::P + S::O + c;
+            double s0 = 0.0, s1 = 0.0;
+            for (int f = 0; f < nf; ++f) {
+                const double2 v = *reinterpret_cast<const double2 *>(p + f * fs);
+                s0 = fma(v.x, v.x, s0);
+                s1 = fma(v.y, v.y, s1);
+            }
+            *reinterpret_cast<double2 *>(ss + row * T + c) =
+                make_double2(fma(ph.kd[GG_G2], s0, -1.0), fma(ph.kd[GG_G2], s1, -1.0));
+        }
+        __syncthreads();
+    }
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + rot;
+    const int c = 2 * (lane % GPR);
+    const int parts = hb / (RG * RR);  // warps that share a field
+    for (int u = warp & 7; u < nf * parts; u += kThreads / 32) {
+        const int f = u / parts, rb = (u % parts) * RG * RR + (lane / GPR) * RR;  // band-local first row
+        const double *p = sm + f * fs + rb * S::P + S::O + c;                     // staged row rb: one above
+        double *out = (double *)a.out[TIER_FP64] + (int64_t)f * a.n + (int64_t)(y0 + r0 + rb) * a.px + x0 + c;
+        auto load = [&](int r, double *w) {
+            const double2 m = *reinterpret_cast<const double2 *>(p + r * S::P);
+            w[0] = p[r * S::P - 1];
+            w[1] = m.x;
+            w[2] = m.y;
+            w[3] = p[r * S::P + 2];
+        };
+        if constexpr (REF) {
+            double w[3][4];
+            load(0, w[0]);
+            load(1, w[1]);
+#pragma unroll
+            for (int i = 0; i < RR; ++i) {
+                const double *rd = w[i % 3], *rc = w[(i + 1) % 3];
+                double *ru = w[(i + 2) % 3];
+                load(i + 2, ru);
+                double v2[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const double e = rc[k + 1];
+                    double s;
+                    if (a.stencil == 0) {
+                        s = __dadd_rn(__dadd_rn(__dadd_rn(rd[k], rd[k + 1]), rd[k + 2]), rc[k]);
+                        s = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(s, rc[k + 2]), ru[k]), ru[k + 1]), ru[k + 2]);
+                        s = __fma_rn(-8.0, e, s);
+                    } else {
+                        s = __fma_rn(-4.0, e, __dadd_rn(__dadd_rn(__dadd_rn(rc[k], rc[k + 2]), rd[k + 1]), ru[k + 1]));
+                    }
+                    const double lap = div_known(s, ph.dxdy, ph.inv_dxdy, ph.dxdy_div);
+                    const double *q = sm + (rb + i + 1) * S::P + S::O + c + k;  // field 0 at this cell
+                    const int b0 = f == 0;                                    // the first other field
+                    double sum = 0.0;
+                    if (b0 < nf) sum = __dmul_rn(q[b0 * fs], q[b0 * fs]);
+                    for (int b = b0 + 1; b < nf; ++b)
+                        if (b != f) sum = __dadd_rn(sum, __dmul_rn(q[b * fs], q[b * fs]));
+                    const double dfd = __dsub_rn(__dadd_rn(__dmul_rn(__dmul_rn(ph.kd[GG_G2], e), sum), cube_rn(e)), e);
+                    v2[k] = __dsub_rn(e, __dmul_rn(ph.kd[GG_DTM], __dsub_rn(dfd, __dmul_rn(ph.grcoef, lap))));
+                }
+                *reinterpret_cast<double2 *>(out + (int64_t)i * a.px) = make_double2(v2[0], v2[1]);
+            }
+        } else {
+            const double m2 = ph.kd[GG_M2], ki = ph.kd[GG_KI], dtm = ph.kd[GG_DTM];
+            // lap: the stencil's sum; g: G at the cell
+            auto update = [&](double e, double lap, double g) {
+                return fma(-dtm, fma(-ki, lap, e * fma(m2, e * e, g)), e);
+            };
+            if (a.stencil == 0) {
+                // h0, h1: row sums of rows i-1, i; e1: the centre values of row i
+                double w[4], h0[2], h1[2], e1[2];
+                auto sums = [&](double *h) {
+                    const double pr = w[1] + w[2];
+                    h[0] = w[0] + pr;
+                    h[1] = pr + w[3];
+                };
+                load(0, w);
+                sums(h0);
+                load(1, w);
+                sums(h1);
+                e1[0] = w[1];
+                e1[1] = w[2];
+#pragma unroll
+                for (int i = 0; i < RR; i += 2) {
+                    double h2[2], h3[2], e2[2], e3[2];
+                    load(i + 2, w);
+                    sums(h2);
+                    e2[0] = w[1];
+                    e2[1] = w[2];
+                    load(i + 3, w);
+                    sums(h3);
+                    e3[0] = w[1];
+                    e3[1] = w[2];
+                    const double2 ga = *reinterpret_cast<const double2 *>(ss + (rb + i) * T + c);
+                    const double2 gb = *reinterpret_cast<const double2 *>(ss + (rb + i + 1) * T + c);
+                    double oa[2], ob[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const double q = h1[k] + h2[k];
+                        oa[k] = update(e1[k], h0[k] + fma(-9.0, e1[k], q), k ? ga.y : ga.x);
+                        ob[k] = update(e2[k], fma(-9.0, e2[k], q) + h3[k], k ? gb.y : gb.x);
+                        h0[k] = h2[k];
+                        h1[k] = h3[k];
+                        e1[k] = e3[k];
+                    }
+                    *reinterpret_cast<double2 *>(out + (int64_t)i * a.px) = make_double2(oa[0], oa[1]);
+                    *reinterpret_cast<double2 *>(out + (int64_t)(i + 1) * a.px) = make_double2(ob[0], ob[1]);
+                }
+            } else {
+#pragma unroll 2
+                for (int i = 0; i < RR; ++i) {
+                    double w[4];
+                    load(i + 1, w);
+                    const double2 up = *reinterpret_cast<const double2 *>(p + i * S::P);
+                    const double2 dn = *reinterpret_cast<const double2 *>(p + (i + 2) * S::P);
+                    const double2 g = *reinterpret_cast<const double2 *>(ss + (rb + i) * T + c);
+                    *reinterpret_cast<double2 *>(out + (int64_t)i * a.px) =
+                        make_double2(update(w[1], fma(-4.0, w[1], (w[0] + w[2]) + (up.x + dn.x)), g.x),
+                                     update(w[2], fma(-4.0, w[2], (w[1] + w[3]) + (up.y + dn.y)), g.y));
+                }
+            }
+        }
+    }
+}
+
+// Rows [row0, row1) of an FP64 tile in bands of hb rows (the whole tile but
+// for a CTA of a split tile), by the whole CTA, in the CTA's staging memory
+// (no copy into it may be in flight).  Out of line: the FP32 path's registers
+// are not shared with it.
+template <int T, bool REF, bool NC = true>
+__device__ __forceinline__ void gg_tile_fp64(const StepArgs &a, float *smf, const uint8_t *nt, int tile, int tx, int ty,
+                                          double *red, int row0, int row1, int hb)
+{
+    double *sm = reinterpret_cast<double *>(smf);
+    double *ss = sm + a.nf * Stage64<T>::field(hb);
+    const int x0 = tx * T, y0 = ty * T;
+    const bool own = (tx + 1) * T > a.nx || (ty + 1) * T > a.ny;  // a ragged grid's edge tile
+    for (int r0 = row0; r0 < row1; r0 += hb) {
+        gg_stage64<T, NC>(a, sm, nt, x0, y0, r0, hb, own);
+        __syncthreads();
+        // the warps' fields rotate with the tile, so that CTAs with fewer
+        // fields than warps load every SM sub-partition's FP64 pipe
+        const int rot = 2 * (tile & 3);
+        if (T == 32 && hb == 16 && a.nf % 8 == 0) gg_band64<T, REF, T == 32 ? 8 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        else if (T == 32 && hb == 16) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        __syncthreads();  // the next band overwrites the staging; the monitor reads the stored tile
+    }
+    if (a.monitor_now) {
+        if (a.monitor_kind == 3) gg_monitor64<T, 3>(a, nt, tile, tx, ty, red);
+        else if (a.monitor_kind == 2) gg_monitor64<T, 2>(a, nt, tile, tx, ty, red);
+        else gg_monitor64<T, 1>(a, nt, tile, tx, ty, red);
+    }
 }
 
 __device__ __forceinline__ __half2 gg_hconst(const Phys &ph, int i)
@@ -518,7 +684,8 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
     // tiers are known, so that its latency overlaps theirs; where the tile
     // turns out FP64 or its neighbourhood mixed, the copies are drained and
     // their data (in-bounds reads of the full-size FP32 store) discarded
-    const bool spec = T == 32 && a.in[TIER_FP32] != nullptr;
+    // (not when every tile is known to be FP64)
+    const bool spec = T == 32 && a.in[TIER_FP32] != nullptr && !a.all64;
     const bool bulk = spec && tm != nullptr && tx >= 1 && ty >= 1 && tx <= a.ntx - 2 && ty <= a.nty - 2;
     if (bulk) {
         if (threadIdx.x == 0) {
@@ -550,11 +717,10 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
     const int tier = a.tier_out[tile];
     __syncthreads();
     if (tier == TIER_FP64) {
-        // the FP64 path reads through L1, not the staging area: the discarded
-        // copies land while it computes, before the CTA exits
-        if (RG && gg_partial_tile(a, T, tx, ty)) gg_tile_fp64_partial<T, REF>(a, ntier, tile, tx, ty, red);
-        else gg_tile_fp64<T, REF>(a, ntier, tile, tx, ty, red);
-        if (spec) spec_done();
+        // the FP64 bands are staged in the same memory: the discarded copies land first
+        if (spec && !spec_done()) return;
+        if (spec && !bulk) __syncthreads();  // every thread's own copies
+        gg_tile_fp64<T, REF, NC>(a, sm, ntier, tile, tx, ty, red, 0, T, gg_fp64_band(T, a.nf));
         return;
     }
     const bool all32 = all_fp32(ntier);
@@ -621,7 +787,7 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
 // measured 18.1 against 15.8 us per adaptive 1024^2 Q=8 step).
 // tm: the tensor map of the step's FP32 input, valid when a.tma_stage.
 template <int T, bool REF, int MK, int HA = 0, bool RG = false>
-__global__ void __launch_bounds__(kThreads, 4) gg_step_kernel(StepArgs a, const __grid_constant__ CUtensorMap tm)
+__global__ void __launch_bounds__(kThreads, 4) gg_step_kernel(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap tm)
 {
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ double red[kThreads / 32];

@@ -88,9 +88,11 @@ __device__ __forceinline__ void gg_tile_pair(const StepArgs &a, float *sm, uint8
     const int tier = a.tier_out[tile];
     __syncthreads();
     if (tier == TIER_FP64) {
-        if (gg_partial_tile(a, T, tx, ty)) gg_tile_fp64_partial<T, REF, PH>(a, ntier, tile, tx, ty, red, f0);
-        else gg_tile_fp64<T, REF, false, PH>(a, ntier, tile, tx, ty, red, f0);
-        if (spec) spec_done();
+        // each CTA takes half of the rows, in bands of 4 (the sums need every
+        // field, and the staging memory is that of half of them)
+        if (spec && !spec_done()) return;
+        __syncthreads();
+        gg_tile_fp64<T, REF>(a, sm, ntier, tile, tx, ty, red, (int)rank * 16, (int)rank * 16 + 16, 4);
         return;
     }
     const bool all32 = all_fp32(ntier);
@@ -110,7 +112,7 @@ __device__ __forceinline__ void gg_tile_pair(const StepArgs &a, float *sm, uint8
     }
     cluster_arrive();  // both stagings complete, visible to the peer
     cluster_wait();
-    float *ss = sm + PH * S::FIELD;  // gg_smem_bytes(32, -1, PH) reserves it
+    float *ss = sm + PH * S::FIELD;  // gg_smem_bytes(32, PH) reserves it
     {
         constexpr int GPR = 8;
         const int row = threadIdx.x / GPR, c = (threadIdx.x % GPR) * 4;
@@ -182,7 +184,7 @@ cudaError_t gg_launch_ens_pair(const EnsLaunch &L, size_t smem, cudaStream_t s)
 }
 
 // staging for a group's member with the most fields
-size_t gg_ens_smem_bytes(int tile, int max_nf) { return gg_smem_bytes(tile, -1, max_nf); }
+size_t gg_ens_smem_bytes(int tile, int max_nf) { return gg_smem_bytes(tile, max_nf); }
 
 #define AMPS_GGE_DISPATCH(MACRO) \
     do {                         \

@@ -3,10 +3,10 @@
 // One launch per step covers every tile; each CTA advances one tile in that
 // tile's own tier.  Half and FP32 tiles stage all Q fields plus a 1-cell halo
 // in shared memory as float (each cell converted from its owner tile's input
-// tier) and store at half/float; FP64 tiles are bound by the FP64 pipes, so
-// they skip the staging and read their neighbourhood straight through L1.
-// Shared memory is therefore sized by the float staging alone.  On monitor
-// steps the epilogue reduces the per-tile metric.
+// tier) and store at half/float; FP64 tiles, bound by the FP64 pipes, stage
+// bands of rows as doubles in the same memory, so that shared memory is sized
+// by the float staging alone.  On monitor steps the epilogue reduces the
+// per-tile metric.
 //
 // Reference: graingrowth/function.h:5-30 (kernel1_pure, launched once per
 // field, graingrowth/purehigh.cu:31-32) and graingrowth/function.h:33-277
@@ -21,89 +21,27 @@
 
 namespace amps {
 
-// All-FP64 step (plain FP64 mode): the FP64 neighbourhood is staged in
-// shared memory, which suits the FP64-pipe-bound arithmetic better than the
-// fused kernel's direct loads.
+// A step whose tiles are all read and written at FP64 (plain FP64 runs, and an
+// adaptive run's first period): a CTA per band of hb rows of a tile, so that
+// the FP64 pipes of all SMs fill evenly.  No tiers and no monitor (monitor
+// steps take the fused kernel).  FP64-pipe bound.  A plain 512^2 Q=8 step (256
+// tiles): 77 us with whole tiles and 18 operations a cell and field, 48 with
+// bands of 8 rows and 10.8 (gg_tile.cuh; the pipe alone needs 38), 51 with
+// bands of 4.
 template <int T, bool REF>
-__global__ void __launch_bounds__(kThreads) gg_step_f64_kernel(StepArgs a)
+__global__ void __launch_bounds__(kThreads, 4) gg_step_f64_kernel(const __grid_constant__ StepArgs a, int hb)
 {
-    using S = Stage<double, T, 1>;
-    constexpr int RPT = T * T / kThreads;
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ double red[kThreads / 32];
-    __shared__ uint8_t ntier[9];
-    double *sm = reinterpret_cast<double *>(smraw);
-    const int tile = blockIdx.x;
-    const int tx = tile % a.ntx, ty = tile / a.ntx;
-    load_neighbour_tiers(a, tx, ty, ntier);
+    double *sm = reinterpret_cast<double *>(smraw), *ss = sm + a.nf * Stage64<T>::field(hb);
+    pdl_trigger();
+    pdl_wait();
+    const int nb = T / hb, tile = blockIdx.x / nb, r0 = (int)(blockIdx.x % nb) * hb;
+    const int x0 = tile % a.ntx * T, y0 = tile / a.ntx * T;
+    gg_stage64<T, true, true>(a, sm, nullptr, x0, y0, r0, hb, false);
     __syncthreads();
-    stage_tile<double, T, 1>(a, sm, ntier, tx, ty, 0, a.nf);
-    __syncthreads();
-    if (gg_partial_tile(a, T, tx, ty)) {  // a ragged grid's edge tile: its wrapped halo
-        patch_ragged<double, T>(a, sm, tx, ty);
-        __syncthreads();
-    }
-    const int col = threadIdx.x % T;
-    const int r0 = (threadIdx.x / T) * RPT;
-    const int c = S::O + col;
-    const int nf = a.nf;
-    const Phys &ph = a.ph;
-    double ssum[RPT];
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) ssum[j] = 0.0;
-    if (!REF)
-        for (int f = 0; f < nf; ++f)
-#pragma unroll
-            for (int j = 0; j < RPT; ++j) {
-                const double v = S::at(sm, f, r0 + j + 1, c);
-                ssum[j] = fma(v, v, ssum[j]);
-            }
-    const int64_t gbase = (int64_t)(ty * T + r0) * a.px + tx * T + col;
-    for (int f = 0; f < nf; ++f) {
-        double w[RPT + 2][3];
-#pragma unroll
-        for (int j = 0; j < RPT + 2; ++j) {
-            w[j][0] = S::at(sm, f, r0 + j, c - 1);
-            w[j][1] = S::at(sm, f, r0 + j, c);
-            w[j][2] = S::at(sm, f, r0 + j, c + 1);
-        }
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-            const double *rd = w[j], *rc = w[j + 1], *ru = w[j + 2];
-            const double e = rc[1];
-            double out;
-            if (REF) {
-                double lap;
-                if (a.stencil == 0)
-                    lap = __ddiv_rn(__dsub_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(
-                                      rd[0], rd[1]), rd[2]), rc[0]), rc[2]), ru[0]), ru[1]), ru[2]),
-                                      __dmul_rn(8.0, e)), ph.dxdy);
-                else
-                    lap = __ddiv_rn(__dsub_rn(__dadd_rn(__dadd_rn(__dadd_rn(rc[0], rc[2]), rd[1]), ru[1]),
-                                              __dmul_rn(4.0, e)), ph.dxdy);
-                double sum = 0.0;
-                bool first = true;
-                for (int b = 0; b < nf; ++b) {
-                    if (b == f) continue;
-                    const double v = S::at(sm, b, r0 + j + 1, c);
-                    const double s2 = __dmul_rn(v, v);
-                    sum = first ? s2 : __dadd_rn(sum, s2);
-                    first = false;
-                }
-                const double dfd = __dsub_rn(__dadd_rn(__dmul_rn(__dmul_rn(2.0 * ph.gamma, e), sum), pow(e, 3.0)), e);
-                out = __dsub_rn(e, __dmul_rn(ph.dt * ph.mobil, __dsub_rn(dfd, __dmul_rn(ph.grcoef, lap))));
-            } else {
-                double s;
-                if (a.stencil == 0) s = (rd[0] + rd[1] + rd[2]) + (rc[0] + rc[2]) + (ru[0] + ru[1] + ru[2]) - 8.0 * e;
-                else s = (rc[0] + rc[2]) + (rd[1] + ru[1]) - 4.0 * e;
-                const double lap = s * ph.inv_dxdy;
-                const double e2 = e * e;
-                const double dfd = e * fma(2.0 * ph.gamma, ssum[j] - e2, e2 - 1.0);
-                out = fma(-(ph.dt * ph.mobil), fma(-ph.grcoef, lap, dfd), e);
-            }
-            ((double *)a.out[TIER_FP64])[(int64_t)f * a.n + gbase + (int64_t)j * a.px] = out;
-        }
-    }
+    const int rot = 2 * ((int)blockIdx.x & 3);  // as in gg_tile_fp64
+    if (T == 32 && a.nf >= 8) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
+    else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot);
 }
 
 // ---- multi-step kernel ---------------------------------------------------------
@@ -164,7 +102,7 @@ __device__ bool flow_wait(const StepArgs &a, const int *done, int tile, int need
 // One CTA per (step, tile) item; a0: the arguments of even steps (counted
 // from the launch's first), a1: of odd ones.
 template <bool REF>
-__global__ void __launch_bounds__(kThreads, 4) gg_flow_kernel(StepArgs a0, StepArgs a1, FlowArgs fl)
+__global__ void __launch_bounds__(kThreads, 4) gg_flow_kernel(const __grid_constant__ StepArgs a0, const __grid_constant__ StepArgs a1, FlowArgs fl)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double red[kThreads / 32];
@@ -189,7 +127,7 @@ __global__ void __launch_bounds__(kThreads, 4) gg_flow_kernel(StepArgs a0, StepA
     }
 }
 
-size_t gg_flow_smem_bytes(int nf) { return gg_smem_bytes(32, -1, nf); }
+size_t gg_flow_smem_bytes(int nf) { return gg_smem_bytes(32, nf); }
 
 cudaError_t gg_prepare_flow(bool ref)
 {
@@ -207,15 +145,16 @@ cudaError_t gg_launch_flow(bool ref, const StepArgs &a0, const StepArgs &a1, con
     return cudaGetLastError();
 }
 
-// tier: TIER_FP64 selects the all-FP64 staged kernel; anything else the fused one.
-size_t gg_smem_bytes(int tile, int tier, int nf)
+size_t gg_smem_bytes(int tile, int nf)
 {
-    if (tier == TIER_FP64)
-        return (size_t)nf * (tile == 32 ? Stage<double, 32, 1>::FIELD : Stage<double, 16, 1>::FIELD) * sizeof(double);
     // 32^2: + the sum-of-squares tile of gg_tile_lo_rows; + 128 bytes to align
-    // the staging for tensor copies (gg_step_kernel)
+    // the staging for tensor copies (gg_step_kernel).  FP64 tiles use the same
+    // memory (gg_fp64_band: 5184 bytes a field and 4096 for their sums).
     if (tile == 32) return ((size_t)nf * Stage<float, 32, 1>::FIELD + 32 * 32) * sizeof(float) + 128;
-    return (size_t)nf * Stage<float, 16, 1>::FIELD * sizeof(float) + 128;
+    const int hb = gg_fp64_band(16, nf);
+    const size_t lo = (size_t)nf * Stage<float, 16, 1>::FIELD * sizeof(float);
+    const size_t hi = ((size_t)nf * Stage64<16>::field(hb) + hb * 16) * sizeof(double);
+    return (lo > hi ? lo : hi) + 128;
 }
 
 template <typename K>
@@ -224,17 +163,24 @@ static cudaError_t launch_pdl(K kernel, int grid, size_t smem, cudaStream_t s, c
     return launch_kernel(kernel, grid, smem, s, true, a, tm);
 }
 
-cudaError_t gg_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, const CUtensorMap *tmp)
+cudaError_t gg_launch(int tile, bool ref, const StepArgs &a, int grid, cudaStream_t s, const CUtensorMap *tmp)
 {
     CUtensorMap none;
     memset(&none, 0, sizeof none);
     const CUtensorMap &tm = tmp ? *tmp : none;
-    const size_t smem = gg_smem_bytes(tile, tier, a.nf);
-#define AMPS_GGL(K, TT)                                                         \
-    do {                                                                        \
-        if (ref) K<TT, true><<<grid, kThreads, smem, s>>>(a);                   \
-        else K<TT, false><<<grid, kThreads, smem, s>>>(a);                      \
-    } while (0)
+    // every tile at FP64: a plain FP64 run (no other tier in use), or a step marked so
+    if (!a.monitor_now && (a.all64 || (a.in[TIER_FP32] == nullptr && a.in[TIER_HALF] == nullptr))) {
+        const int hb = 8;
+        const size_t sm64 = sizeof(double) * (size_t)(tile == 32 ? a.nf * Stage64<32>::field(hb) + hb * 32
+                                                                : a.nf * Stage64<16>::field(hb) + hb * 16);
+        const int n = grid * (tile / hb);
+        if (tile == 32)
+            return ref ? launch_kernel(gg_step_f64_kernel<32, true>, n, sm64, s, true, a, hb)
+                       : launch_kernel(gg_step_f64_kernel<32, false>, n, sm64, s, true, a, hb);
+        return ref ? launch_kernel(gg_step_f64_kernel<16, true>, n, sm64, s, true, a, hb)
+                   : launch_kernel(gg_step_f64_kernel<16, false>, n, sm64, s, true, a, hb);
+    }
+    const size_t smem = gg_smem_bytes(tile, a.nf);
 #define AMPS_GGK(TT, MK)                                                                              \
     do {                                                                                              \
         if (ref) return launch_pdl(gg_step_kernel<TT, true, MK>, grid, smem, s, a, tm);               \
@@ -249,10 +195,7 @@ cudaError_t gg_launch(int tile, int tier, bool ref, const StepArgs &a, int grid,
         default: AMPS_GGK(TT, 3);                                                                     \
         }                                                                                             \
     } while (0)
-    if (tier == TIER_FP64) {
-        if (tile == 32) AMPS_GGL(gg_step_f64_kernel, 32);
-        else AMPS_GGL(gg_step_f64_kernel, 16);
-    } else if (a.nx % tile || a.ny % tile) {
+    if (a.nx % tile || a.ny % tile) {
         return gg_launch_ragged(tile, ref, a, grid, smem, s, tm);  // partial edge tiles (k_gg_ragged.cu)
     } else if (a.half_arith != 0) {
         return gg_launch_half(tile, ref, a, grid, smem, s, tm);  // binary16 half tiles (k_gg_half.cu)
@@ -260,25 +203,22 @@ cudaError_t gg_launch(int tile, int tier, bool ref, const StepArgs &a, int grid,
         if (tile == 32) AMPS_GGM(32);
         else AMPS_GGM(16);
     }
-#undef AMPS_GGL
 #undef AMPS_GGM
 #undef AMPS_GGK
     return cudaGetLastError();
 }
 
-cudaError_t gg_prepare(int tile, int tier, bool ref, int half_arith, bool ragged)
+cudaError_t gg_prepare(int tile, bool ref, int half_arith, bool ragged)
 {
     const int lim = kMaxDynSmem;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    if (tier == TIER_FP64) {
-        if (tile == 32) return ref ? cudaFuncSetAttribute(gg_step_f64_kernel<32, true>, attr, lim)
-                                   : cudaFuncSetAttribute(gg_step_f64_kernel<32, false>, attr, lim);
-        return ref ? cudaFuncSetAttribute(gg_step_f64_kernel<16, true>, attr, lim)
-                   : cudaFuncSetAttribute(gg_step_f64_kernel<16, false>, attr, lim);
-    }
+    cudaError_t e = cudaFuncSetAttribute(gg_step_f64_kernel<32, true>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_f64_kernel<32, false>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_f64_kernel<16, true>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_f64_kernel<16, false>, attr, lim);
+    if (e != cudaSuccess) return e;
     if (half_arith != 0) return gg_prepare_half(tile, ref, half_arith);
     if (ragged) return gg_prepare_ragged(tile, ref);
-    cudaError_t e = cudaSuccess;
 #define AMPS_GGP(TT, MK)                                                                                     \
     if (e == cudaSuccess)                                                                                    \
         e = ref ? cudaFuncSetAttribute(gg_step_kernel<TT, true, MK>, attr, lim)                              \
@@ -302,7 +242,7 @@ cudaError_t gg_prepare(int tile, int tier, bool ref, int half_arith, bool ragged
 // FP64 output) takes the generic staged / direct path.
 template <bool REF>
 __global__ void __launch_bounds__(kThreads, 2)
-    gg_step_tma_kernel(const __grid_constant__ CUtensorMap tm, StepArgs a, int bufstride)
+    gg_step_tma_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ StepArgs a, int bufstride)
 {
     constexpr int T = 32;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -380,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             load_neighbour_tiers(a, tx, ty, ntier);
             __syncthreads();
             if (tier == TIER_FP64) {
-                gg_tile_fp64<T, REF>(a, ntier, t, tx, ty, red);
+                gg_tile_fp64<T, REF>(a, sm, ntier, t, tx, ty, red, 0, T, gg_fp64_band(T, a.nf));
             } else {
                 stage_tile<float, T, 1>(a, sm, ntier, tx, ty, 0, a.nf);
                 __syncthreads();
@@ -394,7 +334,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     // a prefetch is issued only for tiles the loop reaches, so nothing is in flight here
 }
 
-int gg_tma_buffer_floats(int nf) { return ((nf * Stage<float, 32, 1>::FIELD * 4 + 1023) / 1024) * 256; }
+// a buffer holds the fields' FP32 neighbourhoods, or an FP64 tile's band and its sums
+int gg_tma_buffer_floats(int nf) { return ((nf * Stage<float, 32, 1>::FIELD * 4 + 4096 + 1023) / 1024) * 256; }
 size_t gg_tma_smem_bytes(int nf) { return (size_t)2 * gg_tma_buffer_floats(nf) * 4 + 1024; }
 
 cudaError_t gg_launch_tma(bool ref, const CUtensorMap &tm, const StepArgs &a, int grid, cudaStream_t s)
