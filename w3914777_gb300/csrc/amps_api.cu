@@ -168,7 +168,7 @@ static bool encode_field_map(CUtensorMap *tm, void *base, int nx, int ny, int nf
 static size_t tier_size(int t) { return t == TIER_FP64 ? 8 : (t == TIER_FP32 ? 4 : 2); }
 
 // How div_known divides by d.
-static int div_kind(double d)
+static uint8_t div_kind(double d)
 {
     int ex;
     const double m = std::fabs(std::frexp(d, &ex));
@@ -186,6 +186,8 @@ static Phys make_phys(const amps_params &p)
     ph.dxdy = p.dx * p.dy;
     ph.inv_dxdy = 1.0 / ph.dxdy;
     ph.dxdy_div = div_kind(ph.dxdy);
+    ph.dx2_div = div_kind(2.0 * ph.dx);
+    ph.dy2_div = div_kind(2.0 * ph.dy);
     ph.tau = p.tau; ph.epsb = p.epsb; ph.kappa = p.kappa; ph.delta = p.delta; ph.aniso = p.aniso;
     ph.alpha = p.alpha; ph.gama = p.gama; ph.teq = p.teq; ph.theta0 = p.theta0; ph.pi = p.pi; ph.noise = p.noise;
     ph.mobil = p.mobil; ph.grcoef = p.grcoef; ph.gamma = p.gamma;
@@ -213,6 +215,7 @@ static Phys make_phys(const amps_params &p)
         const bool even = ph.aniso >= 2 && ph.aniso <= 16 && ph.aniso == 2 * std::floor(ph.aniso / 2);
         k[KB_MODE] = even ? ph.aniso : 0;
         k[KB_C0] = std::cos(ph.aniso * ph.theta0); k[KB_S0] = std::sin(ph.aniso * ph.theta0);
+        k[KB_DX2] = 2.0 * ph.dx; k[KB_DY2] = 2.0 * ph.dy;
     } else if (p.model == AMPS_GRAINGROWTH) {
         k[GG_G2] = 2.0 * ph.gamma; k[GG_M2] = 1.0 - 2.0 * ph.gamma; k[GG_KI] = ph.grcoef * ph.inv_dxdy;
         k[GG_DTM] = ph.dt * ph.mobil;

@@ -25,7 +25,7 @@ enum { TIER_HALF = 0, TIER_FP32 = 1, TIER_FP64 = 2 };
 // Model constants (double; each kernel rounds them to its compute type).
 struct Phys {
     double dx, dy, dt, dxdy, inv_dxdy;
-    int dxdy_div;  // how div_known divides by dx*dy (enum DivKind)
+    uint8_t dxdy_div, dx2_div, dy2_div;  // how div_known divides by dx*dy, 2dx, 2dy (enum DivKind)
     // Kobayashi
     double tau, epsb, kappa, delta, aniso, alpha, gama, teq, theta0, pi, noise;
     // grain growth
@@ -56,9 +56,9 @@ enum KConst {
     // Kobayashi: 0.5/dx, 0.5/dy, aniso, theta0, epsb, delta, -epsb*aniso*delta,
     // alpha/pi, gama, teq, noise, dt/tau, kappa, dt, 1/dxdy; the anisotropy
     // mode when it is an even integer 2..16 (else 0), cos and sin of
-    // aniso*theta0
+    // aniso*theta0, 2dx, 2dy
     KB_HX, KB_HY, KB_ANISO, KB_THETA0, KB_EPSB, KB_DELTA, KB_ED, KB_M, KB_GAMA, KB_TEQ, KB_NOISE, KB_DTT,
-    KB_KAPPA, KB_DT, KB_INV, KB_MODE, KB_C0, KB_S0,
+    KB_KAPPA, KB_DT, KB_INV, KB_MODE, KB_C0, KB_S0, KB_DX2, KB_DY2,
     // sintering: 1/dxdy, B, 2A, 0.5*coefm, dvol, dvap, dsur, dgrb, dt, 12B, dt*coefl, 0.5*coefk
     SN_INV = 0, SN_B, SN_A2, SN_HCM, SN_DVOL, SN_DVAP, SN_DSUR, SN_DGRB, SN_DT, SN_B12, SN_DTL, SN_HCK,
     // grain growth's FP64 tiles: 2*gamma, 1 - 2*gamma, kappa/(dx*dy), dt*L
@@ -226,12 +226,14 @@ __device__ __forceinline__ double cube_rn(double x)
 // remainders need not be exact, take the general division, as does every x of
 // any other divisor (DIV_GENERAL).
 enum DivKind { DIV_GENERAL, DIV_MUL, DIV_KNOWN };
+// (one copy of the general division, out of line: it is rarely taken)
+__device__ __noinline__ static double div_general(double x, double d) { return __ddiv_rn(x, d); }
 __device__ __forceinline__ double div_known(double x, double d, double inv, int kind)
 {
-    if (kind == DIV_GENERAL) return __ddiv_rn(x, d);
+    if (kind == DIV_GENERAL) return div_general(x, d);
     const double q = __dmul_rn(x, inv);
     if (kind == DIV_MUL || pos_zero(fabs(x))) return q;
-    if ((unsigned)((__double2hiint(x) >> 20 & 0x7ff) - 128) > 1792u) return __ddiv_rn(x, d);
+    if ((unsigned)((__double2hiint(x) >> 20 & 0x7ff) - 128) > 1792u) return div_general(x, d);
     return __fma_rn(__fma_rn(-q, d, x), inv, q);
 }
 

@@ -15,13 +15,11 @@
 namespace amps {
 
 // Seeded uniform noise in [0, 1) of (step a, cell b): SplitMix64's mixing
-// function applied three times, the top 53 bits scaled by 2^-53.
-// noise_u01 split at its per-step key: noise_key(seed, a) is the part that
-// depends on the step only (computed once per tile), noise_u01_k(key, b)
-// the per-cell rest; noise_u01_k(noise_key(seed, a), b) == noise_u01(seed,
-// a, b) bit for bit.  Float: the 53-bit integer rounded once to float and
-// scaled by 2^-53 (exact), which is (float)noise_u01 -- without three FP64
-// operations per cell.
+// function applied three times, the top 53 bits scaled by 2^-53.  noise_key(seed, a)
+// is the part that depends on the step only (computed once per tile),
+// noise_u01_k(key, b) the per-cell rest.  Float: the 53-bit integer rounded
+// once to float and scaled by 2^-53 (exact), which is the double value
+// rounded to float -- without three FP64 operations per cell.
 __device__ __forceinline__ uint64_t noise_mix(uint64_t z)
 {
     z += 0x9E3779B97F4A7C15ull;
@@ -39,11 +37,6 @@ template <> __device__ __forceinline__ float noise_u01_k<float>(uint64_t key, ui
 {
     return __ull2float_rn(noise_mix(key + b) >> 11) * 0x1.0p-53f;
 }
-__device__ __forceinline__ double noise_u01(uint64_t seed, uint64_t a, uint64_t b)
-{
-    return noise_u01_k<double>(noise_key(seed, a), b);
-}
-
 // x != 0 for a double parameter, by an integer test of its bits (no FP64 op)
 __device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
 
@@ -147,6 +140,86 @@ __device__ __forceinline__ void kob_update(const CT *P, const CT *Tm, int sp, co
     tn = fma(kc<CT>(ph, KB_KAPPA), pn - p0, fma(kc<CT>(ph, KB_DT), lt, t0));
 }
 
+// ---- FP64 tiles: per-cell arithmetic, shared by the whole-tile (monitor
+// steps) and the row-band path, so both give the same bits.  Bound by the FP64
+// pipe.  REF: the reference's expression order, every operation rounded on
+// its own; its divisions by dx*dy, 2dx and 2dy are div_known (20 a cell, 3
+// operations each in place of ~10), and cos and sin of the angle share one
+// argument reduction.
+
+// Phase A: a1 = eps*eps'*phi_x, a2 = eps*eps'*phi_y and eps.
+template <bool REF>
+__device__ __forceinline__ void kob_aniso64(const double *P, int ps, const Phys &ph, double &a1, double &a2, double &e)
+{
+    double phx, phy, ed, sn, cs;
+    if (REF) {
+        phx = div_known(__dsub_rn(P[1], P[-1]), ph.kd[KB_DX2], ph.kd[KB_HX], ph.dx2_div);
+        phy = div_known(__dsub_rn(P[ps], P[-ps]), ph.kd[KB_DY2], ph.kd[KB_HY], ph.dy2_div);
+        sincos(__dmul_rn(ph.aniso, __dsub_rn(atan2(phy, phx), ph.theta0)), &sn, &cs);
+        e = __dmul_rn(ph.epsb, __dadd_rn(1.0, __dmul_rn(ph.delta, cs)));
+        ed = __dmul_rn(ph.kd[KB_ED], sn);
+    } else {
+        phx = (P[1] - P[-1]) * ph.kd[KB_HX];
+        phy = (P[ps] - P[-ps]) * ph.kd[KB_HY];
+        sincos(ph.kd[KB_ANISO] * (atan2(phy, phx) - ph.kd[KB_THETA0]), &sn, &cs);
+        e = ph.kd[KB_EPSB] * fma(ph.kd[KB_DELTA], cs, 1.0);
+        ed = ph.kd[KB_ED] * sn;
+    }
+    const double q = __dmul_rn(e, ed);
+    a1 = __dmul_rn(q, phx);
+    a2 = __dmul_rn(q, phy);
+}
+
+// Phase B: phi' and T' from phi and T (P, Tm at the cell, row stride sp) and
+// phase A's arrays at index o (row stride es).
+template <bool REF>
+__device__ __forceinline__ void kob_update64(const double *P, const double *Tm, int sp, const double *a1,
+                                             const double *a2, const double *ep, int o, int es, const Phys &ph,
+                                             uint64_t nkey, int64_t g, double &pn, double &tn)
+{
+    const double p0 = P[0], t0 = Tm[0];
+    if (REF) {
+        // lap: snowflake/function.h:27-28, each term divided separately, left to right
+        auto dv = [&](double v) { return div_known(v, ph.dxdy, ph.inv_dxdy, ph.dxdy_div); };
+        auto lap = [&](const double *c) {
+            double l = dv(c[-1]);
+            l = __dadd_rn(l, dv(c[-2]));
+            l = __dadd_rn(l, dv(c[1]));
+            l = __dadd_rn(l, dv(c[2]));
+            l = __dadd_rn(l, dv(c[-sp]));
+            l = __dadd_rn(l, dv(c[-2 * sp]));
+            l = __dadd_rn(l, dv(c[sp]));
+            l = __dadd_rn(l, dv(c[2 * sp]));
+            return __dsub_rn(l, dv(__dmul_rn(8.0, c[0])));
+        };
+        const double lp = lap(P), lt = lap(Tm);
+        const double term1 = div_known(__dsub_rn(a1[o + es], a1[o - es]), ph.kd[KB_DY2], ph.kd[KB_HY], ph.dy2_div);
+        const double term2 = -div_known(__dsub_rn(a2[o + 1], a2[o - 1]), ph.kd[KB_DX2], ph.kd[KB_HX], ph.dx2_div);
+        const double m = __dmul_rn(ph.kd[KB_M], atan(__dmul_rn(ph.gama, __dsub_rn(ph.teq, t0))));
+        double drive = __dadd_rn(__dsub_rn(p0, 0.5), m);
+        if (nonzero(ph.noise))
+            drive = __dadd_rn(drive, __dmul_rn(ph.noise, __dsub_rn(noise_u01_k<double>(nkey, (uint64_t)g), 0.5)));
+        const double inner = __dadd_rn(__dadd_rn(__dadd_rn(term1, term2), __dmul_rn(__dmul_rn(ep[o], ep[o]), lp)),
+                                       __dmul_rn(__dmul_rn(p0, __dsub_rn(1.0, p0)), drive));
+        pn = __dadd_rn(p0, __dmul_rn(ph.kd[KB_DTT], inner));
+        tn = __dadd_rn(__dadd_rn(t0, __dmul_rn(ph.dt, lt)), __dmul_rn(ph.kappa, __dsub_rn(pn, p0)));
+    } else {
+        auto lap = [&](const double *c) {
+            return ((c[-1] + c[1]) + (c[-2] + c[2]) + (c[-sp] + c[sp]) + (c[-2 * sp] + c[2 * sp]) - 8.0 * c[0]) *
+                   ph.kd[KB_INV];
+        };
+        const double lp = lap(P), lt = lap(Tm);
+        const double term1 = (a1[o + es] - a1[o - es]) * ph.kd[KB_HY];
+        const double term2 = -(a2[o + 1] - a2[o - 1]) * ph.kd[KB_HX];
+        const double m = ph.kd[KB_M] * atan(ph.kd[KB_GAMA] * (ph.kd[KB_TEQ] - t0));
+        double drive = p0 - 0.5 + m;
+        if (nonzero(ph.noise)) drive += ph.kd[KB_NOISE] * (noise_u01_k<double>(nkey, (uint64_t)g) - 0.5);
+        const double inner = term1 + term2 + ep[o] * ep[o] * lp + p0 * (1.0 - p0) * drive;
+        pn = fma(ph.kd[KB_DTT], inner, p0);
+        tn = fma(ph.kd[KB_KAPPA], pn - p0, fma(ph.kd[KB_DT], lt, t0));
+    }
+}
+
 // Threads per Kobayashi tile CTA.  A 512^2 grid is 256 tiles of 32^2, so
 // at 256 threads a tile the step ran one partial wave at ~14 warps per SM,
 // latency-bound; 512 threads a tile double the warps in flight (two cells a
@@ -196,21 +269,14 @@ __device__ __forceinline__ void kob_tile(const StepArgs &a, unsigned char *smraw
             j = bc_map(y0 + j, a.ny, 1) - y0;
         }
         const int r = j + R, cc = i + S::O;
-        const CT pe = S::at(sm, 0, r, cc + 1), pw = S::at(sm, 0, r, cc - 1);
-        const CT pn = S::at(sm, 0, r + 1, cc), ps = S::at(sm, 0, r - 1, cc);
-        CT phx, phy, e, ed;
-        if (REF) {
-            phx = __ddiv_rn(__dsub_rn(pe, pw), 2.0 * ph.dx);
-            phy = __ddiv_rn(__dsub_rn(pn, ps), 2.0 * ph.dy);
-            const double th = atan2((double)phy, (double)phx);
-            const double arg = __dmul_rn(ph.aniso, __dsub_rn(th, ph.theta0));
-            e = __dmul_rn(ph.epsb, __dadd_rn(1.0, __dmul_rn(ph.delta, cos(arg))));
-            ed = __dmul_rn(__dmul_rn(__dmul_rn(-ph.epsb, ph.aniso), ph.delta), sin(arg));
+        const CT *P = &S::at(sm, 0, r, cc);
+        if constexpr (TIER == TIER_FP64) {
+            kob_aniso64<REF>(P, S::P, ph, px[u], py[u], ep[u]);
         } else {
-            kob_aniso<CT, POLY>(&S::at(sm, 0, r, cc), S::P, ph, phx, phy, e, ed);
+            CT phx, phy, e, ed;
+            kob_aniso<CT, POLY>(P, S::P, ph, phx, phy, e, ed);
+            px[u] = phx; py[u] = phy; ep[u] = e; epd[u] = ed;
         }
-        const int o = u;
-        px[o] = phx; py[o] = phy; ep[o] = e; epd[o] = ed;
     }
     __syncthreads();
 
@@ -235,40 +301,8 @@ __device__ __forceinline__ void kob_tile(const StepArgs &a, unsigned char *smraw
         const CT *P = &S::at(sm, 0, r, cc), *Tm = &S::at(sm, 1, r, cc);
         const int64_t g = (int64_t)(y0 + j) * a.nx + x0 + i;
         CT pn, tn;
-        if (REF) {
-            const double d = ph.dxdy;
-            // lap: snowflake/function.h:27-28, each term divided separately, left to right
-            double lp = __ddiv_rn(P[-1], d);
-            lp = __dadd_rn(lp, __ddiv_rn(P[-2], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[1], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[2], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[-S::P], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[-2 * S::P], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[S::P], d));
-            lp = __dadd_rn(lp, __ddiv_rn(P[2 * S::P], d));
-            lp = __dsub_rn(lp, __ddiv_rn(__dmul_rn(8.0, p0), d));
-            double lt = __ddiv_rn(Tm[-1], d);
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[-2], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[1], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[2], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[-S::P], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[-2 * S::P], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[S::P], d));
-            lt = __dadd_rn(lt, __ddiv_rn(Tm[2 * S::P], d));
-            lt = __dsub_rn(lt, __ddiv_rn(__dmul_rn(8.0, t0), d));
-            const int on = o + E, os = o - E, oe = o + 1, ow = o - 1;
-            const double term1 = __ddiv_rn(__dsub_rn(__dmul_rn(__dmul_rn(ep[on], epd[on]), px[on]),
-                                                     __dmul_rn(__dmul_rn(ep[os], epd[os]), px[os])), 2.0 * ph.dy);
-            const double term2 = -__ddiv_rn(__dsub_rn(__dmul_rn(__dmul_rn(ep[oe], epd[oe]), py[oe]),
-                                                      __dmul_rn(__dmul_rn(ep[ow], epd[ow]), py[ow])), 2.0 * ph.dx);
-            const double m = __dmul_rn(ph.alpha / ph.pi, atan(__dmul_rn(ph.gama, __dsub_rn(ph.teq, t0))));
-            double drive = __dadd_rn(__dsub_rn(p0, 0.5), m);
-            if (ph.noise != 0.0)
-                drive = __dadd_rn(drive, __dmul_rn(ph.noise, __dsub_rn(noise_u01(ph.seed, (uint64_t)step, (uint64_t)g), 0.5)));
-            const double inner = __dadd_rn(__dadd_rn(__dadd_rn(term1, term2), __dmul_rn(__dmul_rn(ep[o], ep[o]), lp)),
-                                           __dmul_rn(__dmul_rn(p0, __dsub_rn(1.0, p0)), drive));
-            pn = __dadd_rn(p0, __dmul_rn(ph.dt / ph.tau, inner));
-            tn = __dadd_rn(__dadd_rn(t0, __dmul_rn(ph.dt, lt)), __dmul_rn(ph.kappa, __dsub_rn(pn, p0)));
+        if constexpr (TIER == TIER_FP64) {
+            kob_update64<REF>(P, Tm, S::P, px, py, ep, o, E, ph, nkey, g, pn, tn);
         } else {
             // storage rounding: to nearest, or (half tiles, AMPS_HALF_SR) stochastic
             const bool sr = SR && half && a.half_arith == AMPS_HALF_SR;
@@ -333,6 +367,86 @@ __global__ void __launch_bounds__(kob_threads<T, TIER>()) kob_step_kernel(StepAr
     kob_tile<T, TIER, REF, kob_threads<T, TIER>(), true, true, POLY>(a, smraw, red, ntier, a.list[blockIdx.x]);
 }
 
+// FP64 tiles of a step without the monitor, in bands of br rows, one CTA each
+// (kob_band_rows), so that a grid of few tiles reaches every SM: the FP64 pipe
+// of one SM works 211000 cycles on a 32^2 reference-order tile with general
+// divisions.  phi and T are staged with their 2-cell halo, phase A runs on the
+// band's rows and one more on either side.  Launch order and the programmatic
+// release of the half/FP32 launch as in kob_step_kernel.  A 128 x 96 plain run
+// in the reference's order (12 tiles): 113 us a step as whole tiles with general
+// divisions, 15 in bands; 256^2: 181 and 58; 512^2: 367 and 134; 1024^2: 1275
+// and 473.
+template <int T, bool REF>
+__global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __grid_constant__ StepArgs a, int br)
+{
+    constexpr int W = T + 4, E = T + 2;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ uint8_t ntier[9];
+    pdl_wait();
+    pdl_trigger();
+    const int nb = T / br, items = a.count[TIER_FP64] * nb;
+    if ((int)blockIdx.x >= items) return;
+    double *sp = reinterpret_cast<double *>(smraw), *st = sp + (br + 4) * W;  // phi, T
+    double *a1 = st + (br + 4) * W, *a2 = a1 + (br + 2) * E, *ep = a2 + (br + 2) * E;
+    const Phys &ph = a.ph;
+    const uint64_t nkey = noise_key(ph.seed, (uint64_t)(*a.step_base + a.step_off));
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int tile = a.list[it / nb], ly0 = it % nb * br;
+        const int tx = tile % a.ntx, ty = tile / a.ntx;
+        const int x0 = tx * T, y0 = ty * T;
+        load_neighbour_tiers(a, tx, ty, ntier);
+        __syncthreads();  // (also: the previous item's reads of the staging)
+        stage_band<double, T, 2>(a, sp, ntier, tx, ty, ly0 - 2, br + 4, 0, 2);
+        __syncthreads();
+        // with zero flux an out-of-domain ring cell takes the values of the
+        // cell it mirrors, which lies in the same band
+        for (int u = threadIdx.x; u < (br + 2) * E; u += kThreads) {
+            int ly = ly0 - 1 + u / E, lx = u % E - 1;
+            if (a.bc != 0) {
+                lx = bc_map(x0 + lx, a.nx, 1) - x0;
+                ly = bc_map(y0 + ly, a.ny, 1) - y0;
+            }
+            kob_aniso64<REF>(sp + (ly - ly0 + 2) * W + lx + 2, W, ph, a1[u], a2[u], ep[u]);
+        }
+        __syncthreads();
+        for (int u = threadIdx.x; u < br * T; u += kThreads) {
+            const int i = u % T, j = u / T;
+            const int64_t g = (int64_t)(y0 + ly0 + j) * a.nx + x0 + i;
+            const int c = (j + 2) * W + i + 2;
+            double pn, tn;
+            kob_update64<REF>(sp + c, st + c, W, a1, a2, ep, (j + 1) * E + i + 1, E, ph, nkey, g, pn, tn);
+            store_tier<TIER_FP64>(a, g, pn);
+            store_tier<TIER_FP64>(a, a.n + g, tn);
+        }
+    }
+}
+
+// Rows of a band: the most that still give the grid's tiles four CTAs an SM
+// (a band recomputes phase A on two extra rows: 1.5, 1.25, 1.13 times the
+// tile's rows for bands of 4, 8 and 16).
+static int kob_band_rows(int tile, int ntiles)
+{
+    for (int br = 16; br > (tile == 32 ? 4 : 8); br /= 2)
+        if ((int64_t)ntiles * (tile / br) >= 4 * 152) return br;
+    return tile == 32 ? 4 : 8;
+}
+
+template <int T> static size_t kob_band_smem(int br)
+{
+    return sizeof(double) * (2 * (size_t)(br + 4) * (T + 4) + 3 * (size_t)(br + 2) * (T + 2));
+}
+
+template <int T>
+static cudaError_t kob_launch_band(bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl)
+{
+    // where other tiers are in use the FP64 tiles are few, often none: one CTA
+    // an SM, which loop over the bands
+    const bool mixed = a.in[TIER_HALF] != nullptr || a.in[TIER_FP32] != nullptr;
+    const int br = kob_band_rows(T, mixed ? 0 : grid), n = grid * (T / br), ctas = mixed && n > 152 ? 152 : n;
+    return ref ? launch_kernel(kob_step_f64_band_kernel<T, true>, ctas, kob_band_smem<T>(br), s, pdl, a, br)
+               : launch_kernel(kob_step_f64_band_kernel<T, false>, ctas, kob_band_smem<T>(br), s, pdl, a, br);
+}
+
 // The half and FP32 tiles of a step in one launch (one CTA per tile; FP64
 // tiles are left to the FP64 launch).  Per-tier launches would each cover
 // only part of the grid -- at 512^2 with 32^2 tiles less than one wave apiece
@@ -387,6 +501,7 @@ static cudaError_t kob_launch_tt(int tier, bool ref, const StepArgs &a, int grid
         return poly ? kob_launch_t<T, TIER_FP32, false, true>(a, grid, s, pdl)
                     : kob_launch_t<T, TIER_FP32, false, false>(a, grid, s, pdl);
     default:
+        if (!a.monitor_now) return kob_launch_band<T>(ref, a, grid, s, pdl);
         return ref ? kob_launch_t<T, TIER_FP64, true, false>(a, grid, s, pdl)
                    : kob_launch_t<T, TIER_FP64, false, false>(a, grid, s, pdl);
     }
