@@ -65,6 +65,7 @@ struct amps_handle {
     int *d_log_n = nullptr;
     int64_t *d_step_base = nullptr;
     double *d_stage = nullptr, *d_partials = nullptr, *d_out = nullptr;
+    unsigned *d_count = nullptr;  // arrivals of a launch's blocks (last_block): zero between launches
     double *h_pinned = nullptr;  // nf*n doubles, page-locked
     cudaStream_t own = nullptr, stream = nullptr;
     // private stream on which a handle working on the default stream (which
@@ -252,7 +253,7 @@ static void free_all(amps_handle *h)
         for (int q = 0; q < 2; ++q)
             if (h->store[t][q]) cudaFree(h->store[t][q]);
     void *ps[] = {h->d_tier_prev, h->d_tier_cur, h->d_lists, h->d_order, h->d_counts, h->d_metric, h->d_snap, h->d_stats,
-                  h->d_flags, h->d_log, h->d_log_n, h->d_step_base, h->d_stage, h->d_partials, h->d_out,
+                  h->d_flags, h->d_log, h->d_log_n, h->d_step_base, h->d_stage, h->d_partials, h->d_out, h->d_count,
                   h->d_diag, h->d_sched, h->d_sched_i, h->d_msnap, h->d_mmetric, h->d_snap_keep, h->d_flow,
                   h->d_mu};
     for (void *q : ps)
@@ -333,6 +334,7 @@ extern "C" int amps_create(const amps_params *p, amps_handle **out)
     ALLOC(h->d_stage, sizeof(double) * h->nf * h->n, "staging");
     ALLOC(h->d_partials, sizeof(double) * 2 * 1024, "partials");
     ALLOC(h->d_out, sizeof(double) * 4, "result");
+    ALLOC(h->d_count, sizeof(unsigned), "block counter");
     if (cudaMallocHost((void **)&h->h_pinned, sizeof(double) * h->nf * h->n) != cudaSuccess)
         return fail(AMPS_ERR_ALLOC, "pinned staging");
 #undef ALLOC
@@ -343,6 +345,7 @@ extern "C" int amps_create(const amps_params *p, amps_handle **out)
     cudaMemsetAsync(h->d_stats, 0, sizeof(unsigned long long) * 8, h->stream);
     cudaMemsetAsync(h->d_flags, 0, sizeof(int) * 4, h->stream);
     cudaMemsetAsync(h->d_log_n, 0, sizeof(int), h->stream);
+    cudaMemsetAsync(h->d_count, 0, sizeof(unsigned), h->stream);
     cudaMemsetAsync(h->d_step_base, 0, sizeof(int64_t), h->stream);
     cudaMemsetAsync(h->d_metric, 0, sizeof(double) * h->ntiles, h->stream);
     cudaMemsetAsync(h->d_snap, 0, sizeof(double) * snap, h->stream);
@@ -1075,8 +1078,8 @@ extern "C" int amps_reduce(amps_handle *h, int field, int kind, double *out)
 {
     if (!h || !out || field < 0 || field >= h->nf || kind < 0 || kind > 3) return AMPS_ERR_INVALID;
     Grid g = grid_view(h, h->parity, live_tiers(h));
-    CK(h, reduce_field(g, field, kind, h->d_partials, h->d_out, h->stream));
-    CK(h, cudaMemcpyAsync(h->h_pinned, h->d_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    // the kernel writes its result to the page-locked staging itself
+    CK(h, reduce_field(g, field, kind, h->d_partials, h->d_count, h->h_pinned, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     *out = h->h_pinned[0];
     return AMPS_OK;
@@ -1101,11 +1104,12 @@ extern "C" int amps_compare(amps_handle *h, int field, const double *other, int 
 
 // ------------------------------------------------------------ diagnostics ----
 namespace {
-constexpr int kDiagAcc = 2 * 32 * 32 + 8;  // boundary counters for up to 32 labels
+constexpr int kDiagAcc = 2 * 32 * 32;      // boundary counters for up to 32 labels, zero between calls
+constexpr int kDiagPart = 7 * 1024;        // interface partials
 struct DiagScratch {
-    int *lab, *parent, *box;
+    int *lab, *parent;
     double *field;
-    unsigned long long *acc;
+    unsigned long long *acc, *part;
 };
 }  // namespace
 
@@ -1113,13 +1117,22 @@ static int diag_scratch(amps_handle *h, DiagScratch *d)
 {
     const size_t ints = (size_t)2 * h->n * sizeof(int), dbl = (size_t)h->n * sizeof(double);
     const size_t off_f = (ints + 255) & ~(size_t)255, off_a = off_f + ((dbl + 255) & ~(size_t)255);
-    const size_t total = off_a + kDiagAcc * sizeof(unsigned long long) + 256;
-    if (!h->d_diag) CK(h, cudaMalloc(&h->d_diag, total));
+    const size_t total = off_a + (kDiagAcc + kDiagPart) * sizeof(unsigned long long);
+    if (!h->d_diag) {
+        char *p = nullptr;
+        CK(h, cudaMalloc(&p, total));
+        const cudaError_t e = cudaMemsetAsync(p + off_a, 0, kDiagAcc * sizeof(unsigned long long), h->stream);
+        if (e != cudaSuccess) {
+            cudaFree(p);
+            FAIL(h, AMPS_ERR_CUDA, "diagnostics scratch: %s", cudaGetErrorString(e));
+        }
+        h->d_diag = p;
+    }
     d->lab = (int *)h->d_diag;
     d->parent = d->lab + h->n;
     d->field = (double *)(h->d_diag + off_f);
     d->acc = (unsigned long long *)(h->d_diag + off_a);
-    d->box = (int *)(d->acc + kDiagAcc);
+    d->part = d->acc + kDiagAcc;
     return AMPS_OK;
 }
 
@@ -1151,18 +1164,14 @@ extern "C" int amps_interface(amps_handle *h, int field, double level, double ou
     if (!h || !out || field < 0 || field >= h->nf) return AMPS_ERR_INVALID;
     DiagScratch d;
     if (int r = diag_scratch(h, &d)) return r;
-    if (int r = diag_gather(h)) return r;
     const amps_params &p = h->p;
-    CK(h, diag_interface(h->d_stage + (int64_t)field * h->n, p.nx, p.ny, p.bc, level, d.acc, d.box, h->stream));
-    unsigned long long acc[3];
-    int box[4];
-    CK(h, cudaMemcpyAsync(acc, d.acc, sizeof acc, cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaMemcpyAsync(box, d.box, sizeof box, cudaMemcpyDeviceToHost, h->stream));
+    unsigned long long *res = (unsigned long long *)h->h_pinned;
+    CK(h, diag_interface(grid_view(h, h->parity, live_tiers(h)), field, p.bc, level, d.part, h->d_count, res, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
-    out[0] = (double)acc[0];
-    out[1] = (double)acc[0] * p.dx * p.dy;
-    out[2] = (double)acc[1] * p.dy + (double)acc[2] * p.dx;
-    for (int k = 0; k < 4; ++k) out[3 + k] = acc[0] ? (double)box[k] : -1.0;
+    out[0] = (double)res[0];
+    out[1] = (double)res[0] * p.dx * p.dy;
+    out[2] = (double)res[1] * p.dy + (double)res[2] * p.dx;
+    for (int k = 0; k < 4; ++k) out[3 + k] = res[0] ? (double)(long long)res[3 + k] : -1.0;
     return AMPS_OK;
 }
 
@@ -1186,17 +1195,12 @@ extern "C" int amps_grains(amps_handle *h, double threshold, double level, int64
     if (!h || !out || !order_params(h, &e0, &q, &cf)) return AMPS_ERR_INVALID;
     DiagScratch d;
     if (int r = diag_scratch(h, &d)) return r;
-    if (int r = diag_gather(h)) return r;
     const amps_params &p = h->p;
-    const double *conc = cf >= 0 ? h->d_stage + (int64_t)cf * h->n : nullptr;
-    CK(h, diag_grains(h->d_stage, e0, q, p.nx, p.ny, p.bc, threshold, conc, level, d.lab, d.parent, d.acc,
-                      h->d_flags, h->stream));
-    unsigned long long acc[2];
-    int flag = 0;
-    CK(h, cudaMemcpyAsync(acc, d.acc, sizeof acc, cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaMemcpyAsync(&flag, h->d_flags, sizeof flag, cudaMemcpyDeviceToHost, h->stream));
+    const unsigned long long *acc = (const unsigned long long *)h->h_pinned;
+    CK(h, diag_grains(grid_view(h, h->parity, live_tiers(h)), e0, q, p.bc, threshold, cf, level, d.lab, d.parent, d.acc,
+                      h->d_count, h->d_flags, (unsigned long long *)h->h_pinned, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
-    if (flag & 4) FAIL(h, AMPS_ERR_TIMEOUT, "grain labelling: a union-find walk exceeded the cell count");
+    if (acc[2] & 4) FAIL(h, AMPS_ERR_TIMEOUT, "grain labelling: a union-find walk exceeded the cell count");
     out[0] = (int64_t)acc[0];
     out[1] = (int64_t)acc[1];
     if (mean_area) *mean_area = acc[0] ? (double)acc[1] * p.dx * p.dy / (double)acc[0] : 0.0;
@@ -1209,13 +1213,10 @@ extern "C" int amps_boundary_lengths(amps_handle *h, double level, double *lengt
     if (!h || !lengths || !order_params(h, &e0, &q, &cf) || q > 32) return AMPS_ERR_INVALID;
     DiagScratch d;
     if (int r = diag_scratch(h, &d)) return r;
-    if (int r = diag_gather(h)) return r;
     const amps_params &p = h->p;
-    const double *conc = cf >= 0 ? h->d_stage + (int64_t)cf * h->n : nullptr;
-    CK(h, diag_boundaries(h->d_stage, e0, q, p.nx, p.ny, p.bc, conc, level, d.lab, d.acc, h->stream));
-    std::vector<unsigned long long> acc((size_t)2 * q * q);
-    CK(h, cudaMemcpyAsync(acc.data(), d.acc, acc.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          h->stream));
+    const unsigned long long *acc = (const unsigned long long *)h->h_pinned;
+    CK(h, diag_boundaries(grid_view(h, h->parity, live_tiers(h)), e0, q, p.bc, cf, level, d.acc, h->d_count,
+                          (unsigned long long *)h->h_pinned, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     for (int a = 0; a < q; ++a)
         for (int b = 0; b < q; ++b) {

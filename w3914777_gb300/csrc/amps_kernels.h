@@ -133,20 +133,27 @@ cudaError_t snap_ref_fixup(double *snap, double *keep, const uint8_t *tier, int 
 // Bookkeeping at the end of a period when no classification runs.
 cudaError_t advance_period(int64_t *step_base, int advance, int stat_steps, const int *counts,
                            unsigned long long *stats, cudaStream_t s);
-// FP64 reductions over one field (block partials, then one ordered pass).
-cudaError_t reduce_field(const Grid &g, int field, int kind, double *partials, double *out, cudaStream_t s);
+// FP64 reduction over one field, deterministic.  out: device or page-locked host memory; *counter: zero, and
+// again zero afterwards.
+cudaError_t reduce_field(const Grid &g, int field, int kind, double *partials, unsigned *counter, double *out,
+                         cudaStream_t s);
 cudaError_t compare_field(const Grid &g, int field, const double *other, double *partials, double *out2,
                           cudaStream_t s);
 
-// Diagnostics on row-major FP64 fields (k_diag.cu).  acc/box/lab/parent are
-// device scratch: acc >= max(3, 2*q*q) counters, box 4 ints, lab and parent
-// n ints each; flags bit 2: a union-find walk hit its cap.
-cudaError_t diag_interface(const double *f, int nx, int ny, int bc, double level, unsigned long long *acc, int *box,
-                           cudaStream_t s);
-cudaError_t diag_grains(const double *fields, int e0, int q, int nx, int ny, int bc, double thr, const double *conc,
-                        double clevel, int *lab, int *parent, unsigned long long *acc, int *flags, cudaStream_t s);
-cudaError_t diag_boundaries(const double *fields, int e0, int q, int nx, int ny, int bc, const double *conc,
-                            double clevel, int *lab, unsigned long long *acc, cudaStream_t s);
+// Diagnostics on the tiered state (k_diag.cu).  Results go to `out`, page-locked host memory; *counter is zero and
+// stays so; part / acc / lab / parent are device scratch:
+//   interface: part: 7 counters for each of up to 1024 blocks; out[7] = cells, x- and y-edges, xmin, xmax, ymin, ymax;
+//   grains: acc[2] zero and again zero afterwards, lab and parent n ints each (by storage-independent cell index);
+//     out[3] = grains, labelled cells, flags (bit 2: a union-find walk hit its cap).  Order parameters e0..e0+q-1,
+//     labelled where field cf >= clevel (cf < 0: everywhere);
+//   boundaries: acc[2*q*q] zero and again zero afterwards; out[2*q*q] = x- and y-edges of each label pair (a < b).
+cudaError_t diag_interface(const Grid &g, int field, int bc, double level, unsigned long long *part, unsigned *counter,
+                           unsigned long long *out, cudaStream_t s);
+cudaError_t diag_grains(const Grid &g, int e0, int q, int bc, double thr, int cf, double clevel, int *lab, int *parent,
+                        unsigned long long *acc, unsigned *counter, int *flags, unsigned long long *out,
+                        cudaStream_t s);
+cudaError_t diag_boundaries(const Grid &g, int e0, int q, int bc, int cf, double clevel, unsigned long long *acc,
+                            unsigned *counter, unsigned long long *out, cudaStream_t s);
 // out = {max |a-b|, rms, mean |a-b|}; partials: 3*np doubles
 cudaError_t diag_compare3(const double *a, const double *b, int64_t n, double *partials, int np, double *out,
                           cudaStream_t s);

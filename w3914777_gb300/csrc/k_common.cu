@@ -3,6 +3,7 @@
 // per-tier work lists, and deterministic FP64 reductions.
 #include "../../include/amps.h"
 #include "amps_kernels.h"
+#include "grid_view.cuh"
 
 namespace amps {
 
@@ -73,68 +74,104 @@ cudaError_t gather_fields(const Grid &g, void *dst, int dst_f32, int f0, int nfs
 }
 
 // ------------------------------------------------------ resting monitor ----
-// One CTA per tile: the spatial metric of the current state, and/or the
-// temporal snapshot (same lattice and slots as the fused epilogues).
+// One CTA per tile, a warp per field: the spatial metric of the current state,
+// and/or the temporal snapshot (same lattice and slots as the fused epilogues).
 // diff: the temporal metric against snap (max |state - snap|, the fused
-// temporal monitor's reduction) in place of the range.
-__global__ void monitor_state_kernel(Grid g, int kind, int samples, int mfield, double *metric, double *snap,
-                                     int write_snap, int *flags, int diff)
+// temporal monitor's reduction) in place of the range.  Half and FP32 tiles
+// reduce in float (exact; the range is formed in double).  1024^2 Q=8 FP32, cold: 191 us with a
+// block reduction per field in double, 22 now; sintering's 17 FP64 fields: 396 and 101.
+template <int T>
+__global__ void __launch_bounds__(kThreads) monitor_state_kernel(Grid g, int kind, int samples, int mfield,
+                                                                 double *metric, double *snap, int write_snap,
+                                                                 int *flags, int diff)
 {
-    __shared__ double red[8];
-    const int tile = blockIdx.x;
-    const int T = g.tile;
-    const int tx = tile % g.ntx, ty = tile / g.ntx;
+    __shared__ double red[kThreads / 32];
+    constexpr int NV = T * T / 4;  // four-cell groups of a tile
+    const int tile = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x0 = tile % g.ntx * T, y0 = tile / g.ntx * T, tier = g.tier[tile];
+    // a ragged grid's edge tile: only its cells inside the domain
+    const int vw = min(T, g.nx - x0), vh = min(T, g.ny - y0);
     double result = 0.0;
-    for (int f = 0; f < g.nf; ++f) {
+    bool bad = false;
+    for (int f = warp; f < g.nf; f += kThreads / 32) {
         if (mfield >= 0 && f != mfield) continue;
         const int slot = mfield < 0 ? f : 0;
+        const int64_t fo = (int64_t)f * g.fs;
         double mn = samples ? INFINITY : 1.0, mx = samples && !diff ? -INFINITY : 0.0;
-        int bad = 0;
-        for (int u = threadIdx.x; u < T * T; u += blockDim.x) {
-            const int i = u % T, j = u / T;
-            // a ragged grid's edge tile: only its cells inside the domain
-            if (tx * T + i >= g.nx || ty * T + j >= g.ny) continue;
-            const int64_t c = (int64_t)(ty * T + j) * g.nx + tx * T + i;
-            const int64_t sc = (int64_t)(ty * T + j) * g.px + tx * T + i;  // snapshot slot: storage layout
-            const double v = read_cell(g, f, c);
-            if (!(v == v) || isinf(v)) bad = 1;
-            int si = 0;
-            if (!samples) {
-                int ir = -1, ic = -1;
-                for (int k = 0; k < 4; ++k) {
-                    const int p = kind == 1 ? (k * (T - 1) * 2 + 3) / 6 : T / 8 + k * (T / 4);
-                    if (j == p) ir = k;
-                    if (i == p) ic = k;
-                }
-                si = (ir < 0 || ic < 0) ? -1 : ir * 4 + ic;
-            }
-            if (si < 0) continue;
-            if (diff) {
-                const double r = samples ? snap[(int64_t)slot * g.fs + sc]
-                                         : snap[((int64_t)slot * g.ntx * g.nty + tile) * 16 + si];
-                mx = fmax(mx, fabs(r - v));
+        float mnf = INFINITY, mxf = -INFINITY;
+#pragma unroll 4
+        for (int u = lane; u < NV; u += 32) {
+            const int j = u / (T / 4), i = u % (T / 4) * 4;
+            if (j >= vh || i >= vw) continue;
+            const int64_t sc = (int64_t)(y0 + j) * g.px + x0 + i;  // snapshot slot: storage layout
+            if (tier != TIER_FP64 && !(samples && (diff || write_snap))) {
+                float v[4];
+                load4f(g, tier, fo + sc, v);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i + k < vw) {
+                        bad |= !(fabsf(v[k]) < INFINITY);
+                        mnf = fminf(mnf, v[k]);
+                        mxf = fmaxf(mxf, v[k]);
+                    }
                 continue;
             }
-            mn = fmin(mn, v);
-            mx = fmax(mx, v);
-            if (write_snap) {
-                if (samples) snap[(int64_t)slot * g.fs + sc] = v;
-                else snap[((int64_t)slot * g.ntx * g.nty + tile) * 16 + si] = v;
+            double v[4];
+            load4d(g, tier, fo + sc, v);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (i + k >= vw) continue;
+                bad |= (__double2hiint(v[k]) & 0x7ff00000) == 0x7ff00000;
+                if (!samples) continue;
+                if (diff) {
+                    mx = fmax(mx, fabs(snap[(int64_t)slot * g.fs + sc + k] - v[k]));
+                    continue;
+                }
+                mn = fmin(mn, v[k]);
+                mx = fmax(mx, v[k]);
+                if (write_snap) snap[(int64_t)slot * g.fs + sc + k] = v[k];
             }
         }
-        const double bmx = block_max(mx, red);
-        const double bmn = block_min(mn, red);
-        result = fmax(result, diff ? bmx : bmx - bmn);
-        if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flags, 1);
+        if (samples && tier != TIER_FP64 && !diff && !write_snap) {
+            mn = (double)mnf;
+            mx = (double)mxf;
+        }
+        if (!samples && lane < 16) {  // the 4x4 lattice
+            const int pr = lane / 4, pc = lane % 4;
+            const int j = kind == 1 ? (pr * (T - 1) * 2 + 3) / 6 : T / 8 + pr * (T / 4);
+            const int i = kind == 1 ? (pc * (T - 1) * 2 + 3) / 6 : T / 8 + pc * (T / 4);
+            if (i < vw && j < vh) {
+                const double v = load1d(g, tier, fo + (int64_t)(y0 + j) * g.px + x0 + i);
+                double *sp = snap + ((int64_t)slot * g.ntx * g.nty + tile) * 16 + lane;
+                if (diff) {
+                    mx = fmax(mx, fabs(*sp - v));
+                } else {
+                    mn = fmin(mn, v);
+                    mx = fmax(mx, v);
+                    if (write_snap) *sp = v;
+                }
+            }
+        }
+        mx = warp_max(mx);
+        mn = warp_min(mn);
+        result = fmax(result, diff ? mx : mx - mn);
     }
-    if (threadIdx.x == 0 && metric) metric[tile] = result;
+    if (lane == 0) red[warp] = result;
+    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flags, 1);
+    if (threadIdx.x == 0 && metric) {
+        for (int w = 1; w < kThreads / 32; ++w) result = fmax(result, red[w]);
+        metric[tile] = result;
+    }
 }
 
 cudaError_t monitor_state(const Grid &g, int kind, int samples, int mfield, double *metric, double *snap,
                           int write_snap, int *flags, cudaStream_t s, int diff)
 {
-    monitor_state_kernel<<<g.ntx * g.nty, kThreads, 0, s>>>(g, kind, samples, mfield, metric, snap, write_snap,
-                                                          flags, diff);
+    const int n = g.ntx * g.nty;
+    if (g.tile == 32)
+        monitor_state_kernel<32><<<n, kThreads, 0, s>>>(g, kind, samples, mfield, metric, snap, write_snap, flags, diff);
+    else
+        monitor_state_kernel<16><<<n, kThreads, 0, s>>>(g, kind, samples, mfield, metric, snap, write_snap, flags, diff);
     return cudaGetLastError();
 }
 
@@ -492,51 +529,80 @@ cudaError_t advance_batch(const ClassifyArgs *cs, int count, cudaStream_t s)
 // ---------------------------------------------------------- reductions ----
 constexpr int kRedBlocks = 1024;
 
-__global__ void reduce_partial_kernel(Grid g, int field, int kind, double *partials)
+template <int KIND> __device__ __forceinline__ double fold(double a, double b)
 {
-    __shared__ double red[8];
-    double acc = kind == 1 ? INFINITY : (kind == 2 ? -INFINITY : 0.0);
-    // contiguous chunk per block, fixed order inside: deterministic
-    const int64_t chunk = (g.n + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = blockIdx.x * chunk, hi = min(g.n, lo + chunk);
-    for (int64_t c = lo + threadIdx.x; c < hi; c += blockDim.x) {
-        const double v = read_cell(g, field, c);
-        if (kind == 0) acc += v;
-        else if (kind == 1) acc = fmin(acc, v);
-        else if (kind == 2) acc = fmax(acc, v);
-        else acc += v * v;
+    return KIND == 1 ? fmin(a, b) : (KIND == 2 ? fmax(a, b) : a + b);
+}
+
+// The block's fold of acc in a fixed shape (thread 0 has it): deterministic.
+template <int KIND> __device__ __forceinline__ double block_fold(double acc, double none, double *red)
+{
+    constexpr int NW = kThreads / 32;
+    for (int o = 16; o > 0; o >>= 1) acc = fold<KIND>(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        acc = threadIdx.x < NW ? red[threadIdx.x] : none;
+        for (int o = NW / 2; o > 0; o >>= 1) acc = fold<KIND>(acc, __shfl_xor_sync(0xffffffffu, acc, o));
     }
-    // fixed-shape tree: warp shuffles then warps in order
-    if (kind == 1) acc = block_min(acc, red);
-    else if (kind == 2) acc = block_max(acc, red);
-    else {
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        acc = 0.0;
-        for (int w = 0; w < 8; ++w) acc += red[w];
+    return acc;
+}
+
+// One launch: each block folds its tiles in a fixed order, the last one to
+// finish folds the blocks' partials (out may be page-locked host memory).
+// Bound by the read of the field and the FP64 pipe's share of it (a conversion
+// and an addition a cell), so few blocks that loop: every block's tree costs
+// its threads five FP64 operations.  1024^2 FP32, cold: 91 us as two launches
+// with one thread folding the partials, 12 now.
+template <int T, int KIND>
+__global__ void __launch_bounds__(kThreads) reduce_kernel(Grid g, int field, double *partials, unsigned *counter,
+                                                          double *out)
+{
+    __shared__ double red[kThreads / 32];
+    constexpr int TPT = T * T / 4, PER = kThreads / TPT;  // threads a tile, tiles a block at a time
+    const int l = threadIdx.x % TPT;
+    const double none = KIND == 1 ? INFINITY : (KIND == 2 ? -INFINITY : 0.0);
+    double acc = none;
+#pragma unroll 2
+    for (int t = blockIdx.x * PER + threadIdx.x / TPT; t < g.ntx * g.nty; t += gridDim.x * PER) {
+        const int x = t % g.ntx * T + l % (T / 4) * 4, y = t / g.ntx * T + l / (T / 4);
+        if (x >= g.nx || y >= g.ny) continue;
+        double v[4];
+        load4d(g, g.tier[t], (int64_t)field * g.fs + (int64_t)y * g.px + x, v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (x + k < g.nx) acc = KIND == 3 ? fma(v[k], v[k], acc) : fold<KIND>(acc, v[k]);
     }
+    acc = block_fold<KIND>(acc, none, red);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+    if (!last_block(counter)) return;
+    acc = none;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += kThreads) acc = fold<KIND>(acc, __ldcg(partials + k));
+    acc = block_fold<KIND>(acc, none, red);
+    if (threadIdx.x == 0) *out = acc;
 }
 
-__global__ void reduce_final_kernel(const double *partials, int np, int kind, double *out)
+template <int T>
+static cudaError_t reduce_t(const Grid &g, int field, int kind, double *partials, unsigned *counter, double *out,
+                            cudaStream_t s)
 {
-    if (threadIdx.x != 0) return;
-    double acc = kind == 1 ? INFINITY : (kind == 2 ? -INFINITY : 0.0);
-    for (int k = 0; k < np; ++k) {
-        if (kind == 1) acc = fmin(acc, partials[k]);
-        else if (kind == 2) acc = fmax(acc, partials[k]);
-        else acc += partials[k];
+    constexpr int per = T == 32 ? 1 : 4;
+    const int n = (g.ntx * g.nty + per - 1) / per, blocks = n < 304 ? n : 304;
+    switch (kind) {
+    case 0: reduce_kernel<T, 0><<<blocks, kThreads, 0, s>>>(g, field, partials, counter, out); break;
+    case 1: reduce_kernel<T, 1><<<blocks, kThreads, 0, s>>>(g, field, partials, counter, out); break;
+    case 2: reduce_kernel<T, 2><<<blocks, kThreads, 0, s>>>(g, field, partials, counter, out); break;
+    default: reduce_kernel<T, 3><<<blocks, kThreads, 0, s>>>(g, field, partials, counter, out); break;
     }
-    *out = acc;
+    return cudaGetLastError();
 }
 
-cudaError_t reduce_field(const Grid &g, int field, int kind, double *partials, double *out, cudaStream_t s)
+cudaError_t reduce_field(const Grid &g, int field, int kind, double *partials, unsigned *counter, double *out,
+                         cudaStream_t s)
 {
-    reduce_partial_kernel<<<kRedBlocks, kThreads, 0, s>>>(g, field, kind, partials);
-    reduce_final_kernel<<<1, 32, 0, s>>>(partials, kRedBlocks, kind, out);
-    return cudaGetLastError();
+    return g.tile == 32 ? reduce_t<32>(g, field, kind, partials, counter, out, s)
+                        : reduce_t<16>(g, field, kind, partials, counter, out, s);
 }
 
 __global__ void compare_partial_kernel(Grid g, int field, const double *other, double *partials)
