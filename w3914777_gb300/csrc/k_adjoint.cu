@@ -16,10 +16,11 @@
 // dL/d(delta, K, epsb) into a device double[3].  Each step is ONE fused
 // kernel: a CTA stages its tile plus halo (radius 2 forward, 3 adjoint) in
 // shared memory, computes the intermediates there, and applies the stencil
-// transposes from shared memory.  A transpose gathers over every preimage of
-// the neighbour map, so zero-flux (mirror) boundaries are differentiated
-// exactly: intermediate cotangents are zero outside the domain and the
-// mirrored preimages of a boundary cell are added explicitly.
+// transposes from shared memory.  Zero-flux (mirror) boundaries are
+// differentiated exactly: about a face the mirror makes a symmetric sum over
+// offsets +-k a symmetric matrix, and the transpose of a central difference the
+// negative difference of the odd extension (f(-1) = -f(0)), so a transpose is a
+// stencil on cotangents extended by even or odd reflection.
 //
 // Grain growth: eta_k' = eta_k - dt*L*(dfd_k - kappa*lap eta_k),
 //   dfd_k = eta_k*(eta_k^2 - 1 + 2*gamma*(S - eta_k^2)),  S = sum_j eta_j^2;
@@ -29,6 +30,7 @@
 // (ParamSrc), so a captured CUDA graph of a whole rollout stays valid when
 // they change between calls.
 #include "../../include/amps.h"
+#include "amps_internal.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -36,22 +38,40 @@
 #include <stdio.h>
 
 #include <new>
+#include <type_traits>
 #include <vector>
 
 namespace {
 
+using amps::pdl_trigger;
+using amps::pdl_wait;
+
 constexpr int kAdjThreads = 256;
 constexpr int kMaxAdjSmem = 226 * 1024;  // dynamic shared memory opt-in limit
 
-struct KobAdj {
+// Constants of the Kobayashi kernels in the compute type, rounded on the host.
+template <typename R> struct KobAdj {
     int nx, ny, bc;
-    double dx, dy, dxdy, dt, tau, aniso, theta0, alpha, gama, teq, pi, noise;
+    int mode;          // FP64: the anisotropy mode where it is an even integer 2..16, else 0
+    bool noisy;
     uint64_t seed;
+    double aniso_d;
+    R hx, hy, aniso, theta0, c0, s0;  // 0.5/dx, 0.5/dy, mode, theta0, cos and sin of aniso*theta0
+    R dtt, inv, m, gama, teq, noise, dt, dtinv;  // dt/tau, 1/(dx*dy), alpha/pi, ..., dt/(dx*dy)
+};
+
+// The constants that depend on the differentiable parameters, formed by one
+// thread while the staging loads are in flight: each thread's own kept the
+// FP64 pipe busier than the rest of an FP32 step.
+template <typename R> struct KobPar {
+    R epsb, delta, kappa, ebd, meb, mea, mad;  // ..., -epsb*aniso*delta, -epsb*delta, -epsb*aniso, -aniso*delta
+    uint64_t nkey;                             // the noise's per-step part
 };
 
 struct GgAdj {
     int nx, ny, bc, q, stencil;
-    double dxdy, dt;
+    bool vin, vg, vout;  // 16-byte accesses to the state, the output cotangents, the result
+    double inv, dt;  // 1/(dx*dy)
 };
 
 // The three differentiable parameters and the noise step index: by value,
@@ -83,39 +103,141 @@ __device__ __forceinline__ int nbmap(int i, int n, int bc)
     return i < 0 ? -i - 1 : (i >= n ? 2 * n - i - 1 : i);
 }
 
-// Cells j with M(j + k) = c along one axis of the zero-flux map (direct
-// j = c - k, plus the mirrored preimages of a boundary cell); at most two.
-__device__ __forceinline__ int preimages_noflux(int c, int k, int n, int *j)
+// The driving term's noise: uniform in [0, 1) by (step, cell), as amps_run's.
+__device__ __forceinline__ uint64_t mix64(uint64_t z)
 {
-    int m = 0;
-    if (c - k >= 0 && c - k < n) j[m++] = c - k;
-    if (-1 - c - k >= 0) j[m++] = -1 - c - k;
-    if (2 * n - 1 - c - k < n) j[m++] = 2 * n - 1 - c - k;
-    return m;
+    z += 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+// float: the 53-bit integer rounded once and scaled exactly, the double value rounded to float
+template <typename R> __device__ __forceinline__ R u01(uint64_t nkey, uint64_t cell)
+{
+    const uint64_t v = mix64(nkey + cell) >> 11;
+    if constexpr (sizeof(R) == 4) return __ull2float_rn(v) * 0x1.0p-53f;
+    else return (double)v * 0x1.0p-53;
 }
 
-__device__ __forceinline__ double u01(uint64_t seed, uint64_t a, uint64_t b)
+template <typename R> __device__ __forceinline__ void kob_params(const KobAdj<R> &p, const ParamSrc &ps, KobPar<R> &k)
 {
-    auto mix = [](uint64_t z) {
-        z += 0x9E3779B97F4A7C15ull;
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        return z ^ (z >> 31);
-    };
-    return (double)(mix(mix(seed ^ mix(a)) + b) >> 11) * 0x1.0p-53;
+    double delta, kappa, epsb;
+    int64_t step;
+    load_params(ps, delta, kappa, epsb, step);
+    k.epsb = R(epsb);
+    k.delta = R(delta);
+    k.kappa = R(kappa);
+    k.ebd = R(-epsb * p.aniso_d * delta);
+    k.meb = R(-epsb * delta);
+    k.mea = R(-epsb * p.aniso_d);
+    k.mad = R(-p.aniso_d * delta);
+    k.nkey = mix64(p.seed ^ mix64((uint64_t)step));
 }
 
-template <typename R> __device__ __forceinline__ double block_sum(R v, double *red)
+// cos and sin of the anisotropy angle a = aniso*(atan2(py, px) - theta0).
+// FP64 with an even integer mode: the power of the unit gradient vector (de
+// Moivre's formula; a zero gradient counts as angle 0, as atan2 has it for an
+// even mode), about 40 FP64 operations against ~110 of atan2, sin and cos.
+template <typename R> __device__ __forceinline__ void kob_angle(const KobAdj<R> &p, R px, R py, R &ca, R &sa)
 {
-    double d = (double)v;
+    if constexpr (sizeof(R) == 8) {
+        if (p.mode) {
+            double c = 1.0, s = 0.0;
+            if (px != 0.0 || py != 0.0) {
+                // scaled by a power of two (exact), so that the squares stay in range
+                const int ex = max(__double2hiint(px) >> 20 & 0x7ff, __double2hiint(py) >> 20 & 0x7ff);
+                const double k = __hiloint2double(max(1, min(2046, 2046 - ex)) << 20, 0);
+                const double x = px * k, y = py * k;
+                const double ir = rsqrt(fma(x, x, y * y));
+                c = x * ir;
+                s = y * ir;
+            }
+            double pr = 1.0, pi = 0.0;
+            bool one = true;  // the product so far is 1
+            for (int n = p.mode;;) {
+                if (n & 1) {
+                    const double t = one ? c : fma(pr, c, -pi * s);
+                    pi = one ? s : fma(pr, s, pi * c);
+                    pr = t;
+                    one = false;
+                }
+                n >>= 1;
+                if (!n) break;
+                const double t = fma(c, c, -s * s);
+                s = 2.0 * c * s;
+                c = t;
+            }
+            ca = fma(pr, p.c0, pi * p.s0);
+            sa = fma(pi, p.c0, -pr * p.s0);
+            return;
+        }
+        sincos(p.aniso * (atan2(py, px) - p.theta0), &sa, &ca);
+    } else {
+        sincosf(p.aniso * (atan2f(py, px) - p.theta0), &sa, &ca);
+    }
+}
+
+// s += v for a sum held as s + c: the rounding error of every addition is kept
+// in c (Knuth's exact two-sum), so the sum of a few floats carries twice their
+// precision without touching the FP64 pipe.
+__device__ __forceinline__ void two_sum(float &s, float &c, float v)
+{
+    const float t = s + v, b = t - s;
+    c += (s - (t - b)) + (v - b);
+    s = t;
+}
+
+// The block's sums of three values a thread, each scaled and added into out[k].
+// FP64 addition is what costs (a warp's takes 16 cycles of an SM's pipe): the
+// threads' values meet in shared memory, three warps fold one value each (NT/32 a
+// lane, in two-float arithmetic), and only their trees are FP64.  buf: 3 * NT
+// values of shared memory, free once every thread of the block's NT is here.
+template <int NT, typename R>
+__device__ __forceinline__ void block_sums(R *buf, R a, R b, R c, double sa, double sb, double sc, double *out)
+{
+    __syncthreads();
+    buf[threadIdx.x] = a;
+    buf[NT + threadIdx.x] = b;
+    buf[2 * NT + threadIdx.x] = c;
+    __syncthreads();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w >= 3) return;
+    const R *p = buf + w * NT + lane;
+    double d;
+    if constexpr (sizeof(R) == 4) {
+        float s = p[0], e = 0.f;
+#pragma unroll
+        for (int k = 1; k < NT / 32; ++k) two_sum(s, e, p[32 * k]);
+        d = (double)s + (double)e;
+    } else {
+        d = p[0];
+#pragma unroll
+        for (int k = 1; k < NT / 32; ++k) d += p[32 * k];
+    }
     for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = d;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < kAdjThreads / 32; ++k) s += red[k];
-    return s;
+    if (lane == 0) atomicAdd(&out[w], d * (w == 0 ? sa : (w == 1 ? sb : sc)));
+}
+
+// An asynchronous copy of one element, or of 16 bytes (both sides aligned),
+// from global to shared memory; in flight until gg_stage_wait.
+template <typename R> __device__ __forceinline__ void cp_elem(R *d, const R *g)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(d);
+    if constexpr (sizeof(R) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(g) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa), "l"(g) : "memory");
+}
+template <typename R> __device__ __forceinline__ void cp_16(R *d, const R *g)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(g)
+                 : "memory");
+}
+
+__device__ __forceinline__ void gg_stage_wait()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // A tile of TX x TY cells with a halo of H cells, row-major in shared memory.
@@ -123,62 +245,52 @@ template <int TX, int TY, int H> struct Reg {
     static constexpr int W = TX + 2 * H, HT = TY + 2 * H, N = W * HT;
 };
 
-// Sum over the preimages of cell (cx, cy) for offset (kx, ky) of a shared
-// array holding a region with halo H around the tile at (x0, y0).  Periodic:
-// the one preimage sits at region position c - k (the halo holds wrapped
-// values).  Zero-flux: the array is zero outside the domain, so the direct
-// term is the region value at c - k; mirrored preimages are added.
-template <int TX, int TY, int H, typename R>
-__device__ __forceinline__ R fold_s(const R *a, int x0, int y0, int cx, int cy, int kx, int ky, int nx, int ny,
-                                    int bc)
-{
-    using G = Reg<TX, TY, H>;
-    const int rx = cx - kx - x0 + H, ry = cy - ky - y0 + H;
-    if (bc == 0 || (cx - kx >= 0 && cx - kx < nx && cy - ky >= 0 && cy - ky < ny &&
-                    cx >= 2 && cx < nx - 2 && cy >= 2 && cy < ny - 2))
-        return a[ry * G::W + rx];
-    int jx[3], jy[3];
-    const int mx = preimages_noflux(cx, kx, nx, jx), my = preimages_noflux(cy, ky, ny, jy);
-    R s = R(0);
-    for (int b = 0; b < my; ++b)
-        for (int c = 0; c < mx; ++c) s += a[(jy[b] - y0 + H) * G::W + (jx[c] - x0 + H)];
-    return s;
-}
-
 // ------------------------------------------------------------ Kobayashi ----
+// Threads of a CTA.  32x8 tiles (grids of few tiles, where a step is latency):
+// the widest region in one pass, the forward's 34x10 or the adjoint's 36x12.
+template <int TY> constexpr int kob_fwd_threads() { return TY == 8 ? 352 : 256; }
+template <int TY> constexpr int kob_adj_threads() { return TY == 8 ? 448 : 256; }
+
 // Forward step.  Shared: phi, T over the halo-2 region; eps*epd*px,
 // eps*epd*py and eps over the halo-1 region (at an out-of-domain zero-flux
 // position: the values of the mirrored cell, as the map M looks them up).
+// FP32 bound by latency at moderate sizes, FP64 by the pipe.  us a step,
+// forward / adjoint, before (constants, noise and parameter sums in FP64 per
+// thread, atan2 and sin and cos in FP64) and now: FP32 256^2 12.3/26.7, under
+// 7.4/8.2; 1024^2 65.6/143, 14.0/32.0; FP64 1024^2 398/749, 256/549.
 template <typename R, int TX, int TY>
-__global__ void __launch_bounds__(kAdjThreads) kob_fwd_kernel(KobAdj p, ParamSrc ps, const R *__restrict__ in,
-                                                              R *__restrict__ out)
+__global__ void __launch_bounds__(kob_fwd_threads<TY>()) kob_fwd_kernel(const __grid_constant__ KobAdj<R> p, ParamSrc ps,
+                                                                        const R *__restrict__ in, R *__restrict__ out)
 {
     using R2 = Reg<TX, TY, 2>;
     using R1 = Reg<TX, TY, 1>;
+    constexpr int NT = kob_fwd_threads<TY>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ KobPar<R> k;
     R *sphi = reinterpret_cast<R *>(smem_raw), *sT = sphi + R2::N;
     R *sP1 = sT + R2::N, *sP2 = sP1 + R1::N, *seps = sP2 + R1::N;
-    double delta, kappa, epsb;
-    int64_t step;
-    load_params(ps, delta, kappa, epsb, step);
     const int nx = p.nx, ny = p.ny, bc = p.bc;
     const int64_t n = (int64_t)nx * ny;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     const R *phi = in, *T = in + n;
-    for (int u = threadIdx.x; u < R2::N; u += kAdjThreads) {
+    // launched programmatically after the stream's previous grid: wait for it
+    // (and its writes) before the first global read
+    pdl_trigger();
+    pdl_wait();
+    for (int u = threadIdx.x; u < R2::N; u += NT) {
         const int gx = x0 - 2 + u % R2::W, gy = y0 - 2 + u / R2::W;
-        R a = R(0), b = R(0);
         if (gx < nx + 2 && gy < ny + 2) {
             const int64_t j = (int64_t)nbmap(gy, ny, bc) * nx + nbmap(gx, nx, bc);
-            a = phi[j];
-            b = T[j];
+            cp_elem(sphi + u, phi + j);
+            cp_elem(sT + u, T + j);
+        } else {
+            sphi[u] = sT[u] = R(0);
         }
-        sphi[u] = a;
-        sT[u] = b;
     }
+    if (threadIdx.x == NT - 1) kob_params(p, ps, k);
+    gg_stage_wait();
     __syncthreads();
-    const R aniso = R(p.aniso), th0 = R(p.theta0);
-    for (int u = threadIdx.x; u < R1::N; u += kAdjThreads) {
+    for (int u = threadIdx.x; u < R1::N; u += NT) {
         int gx = x0 - 1 + u % R1::W, gy = y0 - 1 + u / R1::W;
         R P1 = R(0), P2 = R(0), e = R(0);
         if (gx <= nx && gy <= ny) {
@@ -187,11 +299,12 @@ __global__ void __launch_bounds__(kAdjThreads) kob_fwd_kernel(KobAdj p, ParamSrc
                 gy = nbmap(gy, ny, 1);
             }
             const int o = (gy - y0 + 2) * R2::W + (gx - x0 + 2);
-            const R px = (sphi[o + 1] - sphi[o - 1]) * R(0.5 / p.dx);
-            const R py = (sphi[o + R2::W] - sphi[o - R2::W]) * R(0.5 / p.dy);
-            const R a = aniso * (atan2(py, px) - th0);
-            e = R(epsb) * (R(1) + R(delta) * cos(a));
-            const R ed = R(-epsb * p.aniso * delta) * sin(a);
+            const R px = (sphi[o + 1] - sphi[o - 1]) * p.hx;
+            const R py = (sphi[o + R2::W] - sphi[o - R2::W]) * p.hy;
+            R ca, sa;
+            kob_angle(p, px, py, ca, sa);
+            e = k.epsb * (R(1) + k.delta * ca);
+            const R ed = k.ebd * sa;
             P1 = e * ed * px;
             P2 = e * ed * py;
         }
@@ -200,8 +313,7 @@ __global__ void __launch_bounds__(kAdjThreads) kob_fwd_kernel(KobAdj p, ParamSrc
         seps[u] = e;
     }
     __syncthreads();
-    const R dtt = R(p.dt / p.tau), inv = R(1.0 / p.dxdy);
-    for (int u = threadIdx.x; u < TX * TY; u += kAdjThreads) {
+    for (int u = threadIdx.x; u < TX * TY; u += NT) {
         const int i = u % TX, jj = u / TX, gx = x0 + i, gy = y0 + jj;
         if (gx >= nx || gy >= ny) continue;
         const int o = (jj + 2) * R2::W + i + 2, o1 = (jj + 1) * R1::W + i + 1;
@@ -209,88 +321,90 @@ __global__ void __launch_bounds__(kAdjThreads) kob_fwd_kernel(KobAdj p, ParamSrc
         const R ph = sphi[o], t0 = sT[o];
         const R sp = (sphi[o - 1] + sphi[o + 1]) + (sphi[o - 2] + sphi[o + 2]) + (sphi[o - W] + sphi[o + W]) +
                      (sphi[o - 2 * W] + sphi[o + 2 * W]);
-        const R lap = (sp - R(8) * ph) * inv;
+        const R lap = (sp - R(8) * ph) * p.inv;
         const R st = (sT[o - 1] + sT[o + 1]) + (sT[o - 2] + sT[o + 2]) + (sT[o - W] + sT[o + W]) +
                      (sT[o - 2 * W] + sT[o + 2 * W]);
-        const R lapT = (st - R(8) * t0) * inv;
-        const R term1 = (sP1[o1 + R1::W] - sP1[o1 - R1::W]) * R(0.5 / p.dy);
-        const R term2 = -(sP2[o1 + 1] - sP2[o1 - 1]) * R(0.5 / p.dx);
-        const R m = R(p.alpha / p.pi) * atan(R(p.gama) * (R(p.teq) - t0));
+        const R lapT = (st - R(8) * t0) * p.inv;
+        const R term1 = (sP1[o1 + R1::W] - sP1[o1 - R1::W]) * p.hy;
+        const R term2 = -(sP2[o1 + 1] - sP2[o1 - 1]) * p.hx;
+        const R m = p.m * atan(p.gama * (p.teq - t0));
         R drive = ph - R(0.5) + m;
         const int64_t g = (int64_t)gy * nx + gx;
-        if (p.noise != 0.0) drive += R(p.noise) * (R(u01(p.seed, (uint64_t)step, (uint64_t)g)) - R(0.5));
+        if (p.noisy) drive += p.noise * (u01<R>(k.nkey, (uint64_t)g) - R(0.5));
         const R e = seps[o1];
-        const R d = dtt * (term1 + term2 + e * e * lap + ph * (R(1) - ph) * drive);
+        const R d = p.dtt * (term1 + term2 + e * e * lap + ph * (R(1) - ph) * drive);
         out[g] = ph + d;
-        out[n + g] = t0 + R(p.dt) * lapT + R(kappa) * d;
+        out[n + g] = t0 + p.dt * lapT + k.kappa * d;
     }
 }
 
 // Adjoint step.  Shared (halo 3 for phi, 2 for the rest, 1 for the
-// anisotropy cotangents):
-//   phi (R3); mu = gphi' + K gT' and gT' (R2, zero outside a zero-flux domain);
+// anisotropy cotangents), with a zero-flux domain's cotangents extended past
+// its faces -- even where a symmetric sum's transpose reads them, odd where a
+// difference's does:
+//   phi (R3); mu = gphi' + K gT' (R2, odd) and gT' (R2, even);
 //   sin a, cos a, px, py (R2, at out-of-domain positions the mirrored cell's;
 //   eps and epd are rebuilt from them exactly as the forward computes them);
-//   Q = dt/tau*mu*eps^2/dxdy (R2, zero outside); lpx, lpy (R1, zero outside):
-//   the cotangents of px, py including the path through theta = atan2(py, px).
+//   Q = dt/tau*mu*eps^2/dxdy (R2, even); lpx (R1, odd in x), lpy (R1, odd in
+//   y): the cotangents of px, py including the path through theta = atan2(py, px).
 template <typename R, int TX, int TY>
-__global__ void __launch_bounds__(kAdjThreads)
-    kob_adj_kernel(KobAdj p, ParamSrc ps, const R *__restrict__ in, const R *__restrict__ gout, R *__restrict__ gin,
-                   double *__restrict__ gparams)
+__global__ void __launch_bounds__(kob_adj_threads<TY>())
+    kob_adj_kernel(const __grid_constant__ KobAdj<R> p, ParamSrc ps, const R *__restrict__ in,
+                   const R *__restrict__ gout, R *__restrict__ gin, double *__restrict__ gparams)
 {
     using R3 = Reg<TX, TY, 3>;
     using R2 = Reg<TX, TY, 2>;
     using R1 = Reg<TX, TY, 1>;
+    constexpr int NT = kob_adj_threads<TY>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[kAdjThreads / 32];
+    __shared__ KobPar<R> k;
     R *sphi = reinterpret_cast<R *>(smem_raw);
     R *smu = sphi + R3::N, *sgT = smu + R2::N, *ssa = sgT + R2::N, *sca = ssa + R2::N;
     R *spx = sca + R2::N, *spy = spx + R2::N, *sQ = spy + R2::N, *slpx = sQ + R2::N, *slpy = slpx + R1::N;
-    double delta, kappa, epsb;
-    int64_t step;
-    load_params(ps, delta, kappa, epsb, step);
     const int nx = p.nx, ny = p.ny, bc = p.bc;
     const int64_t n = (int64_t)nx * ny;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     const R *phi = in, *T = in + n, *gpo = gout, *gTo = gout + n;
-    const R K = R(kappa);
-    for (int u = threadIdx.x; u < R3::N; u += kAdjThreads) {
+    pdl_trigger();
+    pdl_wait();
+    for (int u = threadIdx.x; u < R3::N; u += NT) {
         const int gx = x0 - 3 + u % R3::W, gy = y0 - 3 + u / R3::W;
-        sphi[u] = (gx < nx + 3 && gy < ny + 3) ? phi[(int64_t)nbmap(gy, ny, bc) * nx + nbmap(gx, nx, bc)] : R(0);
+        if (gx < nx + 3 && gy < ny + 3) cp_elem(sphi + u, phi + (int64_t)nbmap(gy, ny, bc) * nx + nbmap(gx, nx, bc));
+        else sphi[u] = R(0);
     }
-    for (int u = threadIdx.x; u < R2::N; u += kAdjThreads) {
+    for (int u = threadIdx.x; u < R2::N; u += NT) {
         const int gx = x0 - 2 + u % R2::W, gy = y0 - 2 + u / R2::W;
-        const bool dom = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-        R m = R(0), t = R(0);
-        if (gx < nx + 2 && gy < ny + 2 && (bc == 0 || dom)) {
+        if (gx < nx + 2 && gy < ny + 2) {
             const int64_t j = (int64_t)nbmap(gy, ny, bc) * nx + nbmap(gx, nx, bc);
-            t = gTo[j];
-            m = gpo[j] + K * t;
+            cp_elem(sgT + u, gTo + j);
+            cp_elem(smu + u, gpo + j);
+        } else {
+            sgT[u] = smu[u] = R(0);
         }
-        smu[u] = m;
-        sgT[u] = t;
     }
+    if (threadIdx.x == NT - 1) kob_params(p, ps, k);
+    gg_stage_wait();
     __syncthreads();
-    const R aniso = R(p.aniso), th0 = R(p.theta0), dtt = R(p.dt / p.tau), inv = R(1.0 / p.dxdy);
-    const R eb = R(epsb), dl = R(delta), ebd = R(-epsb * p.aniso * delta);
-    auto EPS = [&](R ca) { return eb * (R(1) + dl * ca); };
-    auto EPD = [&](R sa) { return ebd * sa; };
-    // sin a, cos a, px, py and Q over R2
-    for (int u = threadIdx.x; u < R2::N; u += kAdjThreads) {
+    const R K = k.kappa;
+    auto EPS = [&](R ca) { return k.epsb * (R(1) + k.delta * ca); };
+    auto EPD = [&](R sa) { return k.ebd * sa; };
+    // mu, sin a, cos a, px, py and Q over R2
+    for (int u = threadIdx.x; u < R2::N; u += NT) {
         const int gx = x0 - 2 + u % R2::W, gy = y0 - 2 + u / R2::W;
-        R sa = R(0), ca = R(0), px = R(0), py = R(0), q = R(0);
+        R sa = R(0), ca = R(0), px = R(0), py = R(0), q = R(0), mu = R(0);
         if (gx <= nx + 1 && gy <= ny + 1) {
             const bool dom = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
             const int sx = bc == 1 ? nbmap(gx, nx, 1) : gx, sy = bc == 1 ? nbmap(gy, ny, 1) : gy;
             const int o = (sy - y0 + 3) * R3::W + (sx - x0 + 3);
-            px = (sphi[o + 1] - sphi[o - 1]) * R(0.5 / p.dx);
-            py = (sphi[o + R3::W] - sphi[o - R3::W]) * R(0.5 / p.dy);
-            const R a = aniso * (atan2(py, px) - th0);
-            sa = sin(a);
-            ca = cos(a);
+            px = (sphi[o + 1] - sphi[o - 1]) * p.hx;
+            py = (sphi[o + R3::W] - sphi[o - R3::W]) * p.hy;
+            kob_angle(p, px, py, ca, sa);
             const R e = EPS(ca);
-            if (bc == 0 || dom) q = dtt * smu[u] * e * e * inv;
+            mu = smu[u] + K * sgT[u];
+            q = p.dtt * mu * e * e * p.inv;
+            if (bc == 1 && !dom) mu = -mu;
         }
+        smu[u] = mu;
         ssa[u] = sa;
         sca[u] = ca;
         spx[u] = px;
@@ -300,485 +414,418 @@ __global__ void __launch_bounds__(kAdjThreads)
     __syncthreads();
     // anisotropy cotangents over R1; parameter gradients of the tile's own cells
     R gd = R(0), ge = R(0), gk = R(0);
-    for (int u = threadIdx.x; u < R1::N; u += kAdjThreads) {
+    for (int u = threadIdx.x; u < R1::N; u += NT) {
         const int rx = u % R1::W, ry = u / R1::W, gx = x0 - 1 + rx, gy = y0 - 1 + ry;
-        const bool dom = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
         R lpx = R(0), lpy = R(0);
-        if (gx <= nx && gy <= ny && (bc == 0 || dom)) {
-            const int o3 = (ry + 2) * R3::W + rx + 2, o2 = (ry + 1) * R2::W + rx + 1;
+        if (gx <= nx && gy <= ny) {
+            // an out-of-domain zero-flux position: minus the mirrored cell's lpx, lpy
+            const bool dom = gx >= 0 && gx < nx && gy >= 0 && gy < ny, out = bc == 1 && !dom;
+            const int mx = out ? nbmap(gx, nx, 1) - x0 + 1 : rx, my = out ? nbmap(gy, ny, 1) - y0 + 1 : ry;
+            const int o3 = (my + 2) * R3::W + mx + 2, o2 = (my + 1) * R2::W + mx + 1;
             constexpr int W = R3::W;
             const R sp = (sphi[o3 - 1] + sphi[o3 + 1]) + (sphi[o3 - 2] + sphi[o3 + 2]) + (sphi[o3 - W] + sphi[o3 + W]) +
                          (sphi[o3 - 2 * W] + sphi[o3 + 2 * W]);
-            const R lap = (sp - R(8) * sphi[o3]) * inv;
-            const R A = dtt * R(0.5 / p.dy) *
-                        (fold_s<TX, TY, 2>(smu, x0, y0, gx, gy, 0, 1, nx, ny, bc) -
-                         fold_s<TX, TY, 2>(smu, x0, y0, gx, gy, 0, -1, nx, ny, bc));
-            const R B = dtt * R(0.5 / p.dx) *
-                        (fold_s<TX, TY, 2>(smu, x0, y0, gx, gy, -1, 0, nx, ny, bc) -
-                         fold_s<TX, TY, 2>(smu, x0, y0, gx, gy, 1, 0, nx, ny, bc));
-            const R C = dtt * smu[o2] * lap;
+            const R lap = (sp - R(8) * sphi[o3]) * p.inv;
+            const R A = p.dtt * p.hy * (smu[o2 - R2::W] - smu[o2 + R2::W]);
+            const R B = p.dtt * p.hx * (smu[o2 + 1] - smu[o2 - 1]);
+            const R C = p.dtt * smu[o2] * lap;
             const R sa = ssa[o2], ca = sca[o2], px = spx[o2], py = spy[o2];
             const R e = EPS(ca), ed = EPD(sa);
             const R le = A * ed * px + B * ed * py + R(2) * C * e;
             const R led = A * e * px + B * e * py;
             lpx = A * e * ed;
             lpy = B * e * ed;
-            const R la = le * R(-epsb * delta) * sa + led * R(-epsb * p.aniso * delta) * ca;
-            const R lth = aniso * la;
+            const R la = le * k.meb * sa + led * k.ebd * ca;
+            const R lth = p.aniso * la;
             const R r2 = px * px + py * py;
             if (r2 > R(0)) {  // atan2 has no derivative where the gradient vanishes
                 lpx += lth * (-py / r2);
                 lpy += lth * (px / r2);
             }
+            if (out) {
+                lpx = -lpx;
+                lpy = -lpy;
+            }
             if (rx >= 1 && rx <= TX && ry >= 1 && ry <= TY && gx < nx && gy < ny) {
-                gd += le * R(epsb) * ca + led * R(-epsb * p.aniso) * sa;
-                ge += le * (R(1) + R(delta) * ca) + led * R(-p.aniso * delta) * sa;
+                gd += le * k.epsb * ca + led * k.mea * sa;
+                ge += le * (R(1) + k.delta * ca) + led * k.mad * sa;
             }
         }
         slpx[u] = lpx;
         slpy[u] = lpy;
     }
     __syncthreads();
-    for (int u = threadIdx.x; u < TX * TY; u += kAdjThreads) {
+    for (int u = threadIdx.x; u < TX * TY; u += NT) {
         const int i = u % TX, jj = u / TX, gx = x0 + i, gy = y0 + jj;
         if (gx >= nx || gy >= ny) continue;
-        const int o3 = (jj + 3) * R3::W + i + 3, o2 = (jj + 2) * R2::W + i + 2;
-        constexpr int W = R3::W;
+        const int o3 = (jj + 3) * R3::W + i + 3, o2 = (jj + 2) * R2::W + i + 2, o1 = (jj + 1) * R1::W + i + 1;
+        constexpr int W = R3::W, W2 = R2::W;
         // transposes: radius-2 cross of Q (eps^2 lap phi) and of gT' (lap T)
         R lq = -R(8) * sQ[o2], lt = -R(8) * sgT[o2];
-        const int off[4] = {-2, -1, 1, 2};
+        const int off[4] = {2, 1, -1, -2};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            lq += fold_s<TX, TY, 2>(sQ, x0, y0, gx, gy, off[k], 0, nx, ny, bc) +
-                  fold_s<TX, TY, 2>(sQ, x0, y0, gx, gy, 0, off[k], nx, ny, bc);
-            lt += fold_s<TX, TY, 2>(sgT, x0, y0, gx, gy, off[k], 0, nx, ny, bc) +
-                  fold_s<TX, TY, 2>(sgT, x0, y0, gx, gy, 0, off[k], nx, ny, bc);
+        for (int j = 0; j < 4; ++j) {
+            lq += sQ[o2 + off[j]] + sQ[o2 + off[j] * W2];
+            lt += sgT[o2 + off[j]] + sgT[o2 + off[j] * W2];
         }
-        const R dpx = (fold_s<TX, TY, 1>(slpx, x0, y0, gx, gy, 1, 0, nx, ny, bc) -
-                       fold_s<TX, TY, 1>(slpx, x0, y0, gx, gy, -1, 0, nx, ny, bc)) *
-                      R(0.5 / p.dx);
-        const R dpy = (fold_s<TX, TY, 1>(slpy, x0, y0, gx, gy, 0, 1, nx, ny, bc) -
-                       fold_s<TX, TY, 1>(slpy, x0, y0, gx, gy, 0, -1, nx, ny, bc)) *
-                      R(0.5 / p.dy);
+        const R dpx = (slpx[o1 - 1] - slpx[o1 + 1]) * p.hx;
+        const R dpy = (slpy[o1 - R1::W] - slpy[o1 + R1::W]) * p.hy;
         // the forward increment d = phi' - phi at this cell (for dL/dK)
         auto P1 = [&](int o) { return EPS(sca[o]) * EPD(ssa[o]) * spx[o]; };
         auto P2 = [&](int o) { return EPS(sca[o]) * EPD(ssa[o]) * spy[o]; };
-        const R term1 = (P1(o2 + R2::W) - P1(o2 - R2::W)) * R(0.5 / p.dy);
-        const R term2 = -(P2(o2 + 1) - P2(o2 - 1)) * R(0.5 / p.dx);
+        const R term1 = (P1(o2 + W2) - P1(o2 - W2)) * p.hy;
+        const R term2 = -(P2(o2 + 1) - P2(o2 - 1)) * p.hx;
         const R ph = sphi[o3];
         const R sp = (sphi[o3 - 1] + sphi[o3 + 1]) + (sphi[o3 - 2] + sphi[o3 + 2]) + (sphi[o3 - W] + sphi[o3 + W]) +
                      (sphi[o3 - 2 * W] + sphi[o3 + 2 * W]);
-        const R lap = (sp - R(8) * ph) * inv;
+        const R lap = (sp - R(8) * ph) * p.inv;
         const int64_t g = (int64_t)gy * nx + gx;
         const R t0 = T[g];
-        const R m = R(p.alpha / p.pi) * atan(R(p.gama) * (R(p.teq) - t0));
+        const R m = p.m * atan(p.gama * (p.teq - t0));
         R drive = ph - R(0.5) + m;
-        if (p.noise != 0.0) drive += R(p.noise) * (R(u01(p.seed, (uint64_t)step, (uint64_t)g)) - R(0.5));
+        if (p.noisy) drive += p.noise * (u01<R>(k.nkey, (uint64_t)g) - R(0.5));
         const R e = EPS(sca[o2]);
-        const R d = dtt * (term1 + term2 + e * e * lap + ph * (R(1) - ph) * drive);
+        const R d = p.dtt * (term1 + term2 + e * e * lap + ph * (R(1) - ph) * drive);
         const R mu = smu[o2];
         const R dg = (R(1) - R(2) * ph) * drive + ph * (R(1) - ph);
-        gin[g] = gpo[g] + dtt * mu * dg + lq + dpx + dpy;
-        const R z = R(p.gama) * (R(p.teq) - t0);
-        const R dm = R(p.alpha / p.pi) * (-R(p.gama)) / (R(1) + z * z);
-        gin[n + g] = gTo[g] + R(p.dt * inv) * lt + dtt * mu * ph * (R(1) - ph) * dm;
-        gk += gTo[g] * d;
+        const R gT = sgT[o2];
+        gin[g] = gpo[g] + p.dtt * mu * dg + lq + dpx + dpy;
+        const R z = p.gama * (p.teq - t0);
+        const R dm = p.m * (-p.gama) / (R(1) + z * z);
+        gin[n + g] = gT + p.dtinv * lt + p.dtt * mu * ph * (R(1) - ph) * dm;
+        gk += gT * d;
     }
-    const double sd = block_sum(gd, red);
-    const double sk = block_sum(gk, red);
-    const double se = block_sum(ge, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(&gparams[0], sd);
-        atomicAdd(&gparams[1], sk);
-        atomicAdd(&gparams[2], se);
-    }
+    block_sums<NT>(sphi, gd, gk, ge, 1.0, 1.0, 1.0, gparams);  // (the staging is over 3 * NT values)
 }
 
 // --------------------------------------------------------- grain growth ----
-// One cell per thread on a kGX x kGY tile; every field of the tile plus a
-// halo of one staged in shared memory (field-major).
-constexpr int kGX = 32, kGY = 8;
-using GReg = Reg<kGX, kGY, 1>;
-
-// One element from global to shared memory by an asynchronous copy (the
-// copies of all rows stay in flight until gg_stage_wait).
-template <typename R> __device__ __forceinline__ void cp_elem(R *d, const R *g)
-{
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(d);
-    if constexpr (sizeof(R) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(g) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa), "l"(g) : "memory");
-}
-
-__device__ __forceinline__ void gg_stage_wait()
-{
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-// Stage q fields of f (row-major [q][n]) over the halo-1 region, one warp
-// per region row (a coalesced copy of the row's kGX interior cells, two
-// lanes for its halo cells); complete after gg_stage_wait.  zero_out:
-// zero-flux cotangents are zero outside the domain (the transpose adds the
-// mirrored preimages itself).
-template <typename R>
-__device__ __forceinline__ void gg_stage(R *s, const R *f, int q, int x0, int y0, const GgAdj &p, bool zero_out)
-{
-    static_assert(kGX == 32, "one lane per interior column");
-    const int64_t n = (int64_t)p.nx * p.ny;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool zf = zero_out && p.bc == 1;
-    for (int rr = warp; rr < q * GReg::HT; rr += kAdjThreads / 32) {
-        const int k = rr / GReg::HT, ry = rr - k * GReg::HT;
-        const int gy = y0 - 1 + ry;
-        const bool rowok = gy <= p.ny && !(zf && (gy < 0 || gy >= p.ny));
-        const R *row = f + k * n + (int64_t)(rowok ? nbmap(gy, p.ny, p.bc) : 0) * p.nx;
-        R *dst = s + k * GReg::N + ry * GReg::W;
-        const int gx = x0 + lane;
-        if (rowok && gx <= p.nx && !(zf && gx >= p.nx))
-            cp_elem(dst + 1 + lane, row + nbmap(gx, p.nx, p.bc));
-        else
-            dst[1 + lane] = R(0);
-        if (lane < 2) {
-            const int hx = lane == 0 ? x0 - 1 : x0 + kGX;
-            R *d = dst + (lane == 0 ? 0 : GReg::W - 1);
-            if (rowok && hx <= p.nx && !(zf && (hx < 0 || hx >= p.nx)))
-                cp_elem(d, row + nbmap(hx, p.nx, p.bc));
-            else
-                *d = R(0);
-        }
+// One 32 x TY tile per CTA (any sides, both boundaries): every field (the
+// adjoint: and every output cotangent) with a 1-cell halo staged by
+// asynchronous copies, the per-cell sums S = sum e^2 (and P = sum g e) formed
+// once into shared tiles, then a warp advances one field, a lane sweeping
+// TY/4 rows x 4 cells with running row sums (with fewer than 8 fields two or
+// four warps share a field's rows).
+//
+// The zero-flux map mirrors about the domain's faces (-1 -> 0, n -> n-1).  On
+// each axis the three-point sum is then a symmetric matrix (the mirrored
+// neighbour adds to the diagonal), so both stencils' Laplacians are symmetric
+// for either boundary: the adjoint applies the forward Laplacian to the
+// cotangents, staged through the same map.
+//
+// FP32 bound: issue slots and the latency of one partial wave at moderate
+// sizes, so TY = 16 (four adjoint CTAs an SM at 8 fields, against two of 32
+// rows); FP64 bound: the FP64 pipe, hence the shared row sums and the factored
+// formulas (about 11 operations a cell and field forward, 28 adjoint, where
+// the direct forms take 18 and 45).  us a step, forward / adjoint, before and now:
+// FP32 1024^2 Q=8 periodic 22.6/51.2, 13.7/39.3; 605x443 Q=8 zero-flux 14.6/44.3,
+// 8.4/14.3; FP64 1024^2 Q=8 271/739, 189/503.
+// The kernels' constants, formed by one thread while the copies are in flight
+// (each thread's own would keep the FP64 pipe busier than the step itself).
+template <typename R> struct GgConst {
+    R dtm, g2, g4, m2, ki;      // dt*L, 2 gamma, 4 gamma, 1 - 2 gamma, kappa/(dx*dy)
+    double sl, sk, sg;          // scales of the parameter sums
+    __device__ void set(const GgAdj &p, double mobil, double grcoef, double gamma)
+    {
+        dtm = R(p.dt * mobil);
+        g2 = R(2.0 * gamma);
+        g4 = R(4.0 * gamma);
+        m2 = R(1.0 - 2.0 * gamma);
+        ki = R(grcoef * p.inv);
+        sl = -p.dt;
+        sk = p.dt * mobil * p.inv;
+        sg = -2.0 * p.dt * mobil;
     }
-}
-
-// 8-neighbour (graingrowth/function.h:20) or 5-point Laplacian at region offset o, / dxdy
-template <typename R> __device__ __forceinline__ R gg_lap_s(const R *s, int o, int stencil, R inv)
-{
-    constexpr int W = GReg::W;
-    R v;
-    if (stencil == 0)
-        v = s[o - W - 1] + s[o - W] + s[o - W + 1] + s[o - 1] + s[o + 1] + s[o + W - 1] + s[o + W] + s[o + W + 1] -
-            R(8) * s[o];
-    else
-        v = s[o - 1] + s[o + 1] + s[o - W] + s[o + W] - R(4) * s[o];
-    return v * inv;
-}
-
-// transpose of gg_lap_s at cell (gx, gy) (exact for both boundary maps)
-template <typename R>
-__device__ __forceinline__ R gg_lap_t_s(const R *s, int o, int x0, int y0, int gx, int gy, const GgAdj &p, R inv)
-{
-    // the stencil is symmetric: where no mirrored preimage exists (periodic
-    // grids, and cells off a zero-flux edge) its transpose is itself
-    if (p.bc == 0 || (gx >= 1 && gx < p.nx - 1 && gy >= 1 && gy < p.ny - 1)) return gg_lap_s(s, o, p.stencil, inv);
-    R v;
-    if (p.stencil == 0) {
-        v = -R(8) * s[o];
-        for (int ky = -1; ky <= 1; ++ky)
-            for (int kx = -1; kx <= 1; ++kx)
-                if (kx || ky) v += fold_s<kGX, kGY, 1>(s, x0, y0, gx, gy, kx, ky, p.nx, p.ny, p.bc);
-    } else {
-        v = fold_s<kGX, kGY, 1>(s, x0, y0, gx, gy, -1, 0, p.nx, p.ny, p.bc) +
-            fold_s<kGX, kGY, 1>(s, x0, y0, gx, gy, 1, 0, p.nx, p.ny, p.bc) +
-            fold_s<kGX, kGY, 1>(s, x0, y0, gx, gy, 0, -1, p.nx, p.ny, p.bc) +
-            fold_s<kGX, kGY, 1>(s, x0, y0, gx, gy, 0, 1, p.nx, p.ny, p.bc) - R(4) * s[o];
-    }
-    return v * inv;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kAdjThreads) gg_fwd_kernel(GgAdj p, ParamSrc ps, const R *__restrict__ eta,
-                                                             R *__restrict__ out)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *se = reinterpret_cast<R *>(smem_raw);
-    double mobil, grcoef, gamma;
-    int64_t step;
-    load_params(ps, mobil, grcoef, gamma, step);
-    const int x0 = blockIdx.x * kGX, y0 = blockIdx.y * kGY;
-    gg_stage(se, eta, p.q, x0, y0, p, false);
-    gg_stage_wait();
-    __syncthreads();
-    const int i = threadIdx.x % kGX, j = threadIdx.x / kGX, gx = x0 + i, gy = y0 + j;
-    if (gx >= p.nx || gy >= p.ny) return;
-    const int64_t n = (int64_t)p.nx * p.ny, g = (int64_t)gy * p.nx + gx;
-    const int o = (j + 1) * GReg::W + i + 1;
-    R S = R(0);
-    for (int k = 0; k < p.q; ++k) S += se[k * GReg::N + o] * se[k * GReg::N + o];
-    const R dtm = R(p.dt * mobil), g2 = R(2.0 * gamma), kap = R(grcoef), inv = R(1.0 / p.dxdy);
-    for (int k = 0; k < p.q; ++k) {
-        const R *sk = se + k * GReg::N;
-        const R e = sk[o], e2 = e * e;
-        const R dfd = e * (e2 - R(1) + g2 * (S - e2));
-        out[k * n + g] = e - dtm * (dfd - kap * gg_lap_s(sk, o, p.stencil, inv));
-    }
-}
-
-// input cotangents of all q fields; adds dL/d(L, kappa, gamma) into gparams
-template <typename R>
-__global__ void __launch_bounds__(kAdjThreads) gg_adj_kernel(GgAdj p, ParamSrc ps, const R *__restrict__ eta,
-                                                             const R *__restrict__ gout, R *__restrict__ gin,
-                                                             double *__restrict__ gparams)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[kAdjThreads / 32];
-    R *se = reinterpret_cast<R *>(smem_raw), *sg = se + p.q * GReg::N;
-    double mobil, grcoef, gamma;
-    int64_t step;
-    load_params(ps, mobil, grcoef, gamma, step);
-    const int x0 = blockIdx.x * kGX, y0 = blockIdx.y * kGY;
-    gg_stage(se, eta, p.q, x0, y0, p, false);
-    gg_stage(sg, gout, p.q, x0, y0, p, true);
-    gg_stage_wait();
-    __syncthreads();
-    const int i = threadIdx.x % kGX, j = threadIdx.x / kGX, gx = x0 + i, gy = y0 + j;
-    R gl = R(0), gkap = R(0), ggam = R(0);
-    if (gx < p.nx && gy < p.ny) {
-        const int64_t n = (int64_t)p.nx * p.ny, g = (int64_t)gy * p.nx + gx;
-        const int o = (j + 1) * GReg::W + i + 1;
-        R S = R(0), P = R(0);
-        for (int k = 0; k < p.q; ++k) {
-            const R e = se[k * GReg::N + o];
-            S += e * e;
-            P += sg[k * GReg::N + o] * e;
-        }
-        const R dt = R(p.dt), dtm = R(p.dt * mobil), gm = R(gamma), kap = R(grcoef), inv = R(1.0 / p.dxdy);
-        for (int k = 0; k < p.q; ++k) {
-            const R *ek = se + k * GReg::N, *gk_s = sg + k * GReg::N;
-            const R e = ek[o], e2 = e * e, gk = gk_s[o];
-            const R jac = R(3) * e2 - R(1) + R(2) * gm * (S - e2);  // d dfd_k / d eta_k
-            gin[k * n + g] = gk - dtm * (gk * jac + R(4) * gm * e * (P - gk * e)) +
-                             dtm * kap * gg_lap_t_s(gk_s, o, x0, y0, gx, gy, p, inv);
-            const R lap = gg_lap_s(ek, o, p.stencil, inv);
-            const R dfd = e * (e2 - R(1) + R(2) * gm * (S - e2));
-            gl += gk * (-dt) * (dfd - kap * lap);
-            gkap += gk * dtm * lap;
-            ggam += gk * (-dtm) * R(2) * e * (S - e2);
-        }
-    }
-    const double a = block_sum(gl, red);
-    const double b = block_sum(gkap, red);
-    const double c = block_sum(ggam, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(&gparams[0], a);
-        atomicAdd(&gparams[1], b);
-        atomicAdd(&gparams[2], c);
-    }
-}
-
-// ---- grain growth, periodic grids, 32x32 tiles ----------------------------
-// The forward step and its adjoint for periodic grids whose sides are
-// multiples of 32 (the Laplacian is then its own transpose): every field of a
-// 32x32 tile plus its halo staged by asynchronous copies in a 16-byte-aligned
-// row layout, the per-cell sums (S = sum e^2; the adjoint's P = sum g e)
-// formed once into shared tiles, then each warp advances one field at a
-// time, a lane sweeping 8 rows x 4 cells with a 3-row register window (the
-// grain-growth step kernel's layout).  The neighbour sums keep gg_lap_s's
-// left-to-right order, so the forward results are gg_fwd_kernel's.
-constexpr int kG32Rows = 8;  // rows per lane
-
-template <typename R> struct G32 {
-    static constexpr int T = 32, O = 16 / (int)sizeof(R) >= 1 ? 16 / (int)sizeof(R) : 1;
-    static constexpr int P = T + 2 * O, ROWS = T + 2, FIELD = ROWS * P;
-    static size_t smem(int nfields, int sums) { return sizeof(R) * ((size_t)nfields * FIELD + (size_t)sums * T * T); }
 };
 
-// Stage q fields (periodic) of tile (tx, ty): one warp per staged row.
-template <typename R>
-__device__ __forceinline__ void gg_stage32(R *s, const R *f, int q, int tx, int ty, const GgAdj &p)
+template <typename R, int TY> struct G32 {
+    static constexpr int T = 32, O = 16 / (int)sizeof(R), P = T + 2 * O, ROWS = TY + 2, FIELD = ROWS * P;
+    static size_t smem(int nfields, int sums) { return sizeof(R) * ((size_t)nfields * FIELD + (size_t)sums * TY * T); }
+};
+
+// Stage q fields of f (row-major [q][ny][nx]) over the tile at (x0, y0) and its
+// halo through the boundary map; cells past the one that a last valid cell
+// reads are zero.  A thread owns a slot -- a 16-byte chunk, a halo cell -- of
+// every field.  vec: nx * sizeof(R) and the base are multiples of 16 bytes.
+template <typename R, int TY>
+__device__ __forceinline__ void gg_stage32(R *s, const R *f, int q, int x0, int y0, const GgAdj &p, bool vec)
 {
-    using L = G32<R>;
+    using L = G32<R, TY>;
+    constexpr int V = 16 / (int)sizeof(R), CH = L::T / V, UI = L::ROWS * CH;
     const int64_t n = (int64_t)p.nx * p.ny;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x0 = tx * L::T;
-    for (int rr = warp; rr < q * L::ROWS; rr += kAdjThreads / 32) {
-        const int k = rr / L::ROWS, ry = rr - k * L::ROWS;
-        int gy = ty * L::T - 1 + ry;
-        gy = gy < 0 ? gy + p.ny : (gy >= p.ny ? gy - p.ny : gy);
-        const R *row = f + k * n + (int64_t)gy * p.nx;
-        R *dst = s + k * L::FIELD + ry * L::P + L::O;
-        cp_elem(dst + lane, row + x0 + lane);
-        if (lane < 2) {
-            int hx = lane == 0 ? x0 - 1 : x0 + L::T;
-            hx = hx < 0 ? hx + p.nx : (hx >= p.nx ? hx - p.nx : hx);
-            cp_elem(dst + (lane == 0 ? -1 : L::T), row + hx);
+    const int units = vec ? UI + L::ROWS * 2 : L::ROWS * (L::T + 2);
+    for (int u = threadIdx.x; u < units; u += kAdjThreads) {
+        int ry, c;  // staged row, tile column
+        bool chunk = false;
+        if (vec && u < UI) {
+            ry = u / CH;
+            c = u % CH * V;
+            chunk = x0 + c < p.nx;
+        } else if (vec) {
+            ry = (u - UI) / 2;
+            c = (u - UI) % 2 ? L::T : -1;
+        } else {
+            ry = u / (L::T + 2);
+            c = u % (L::T + 2) - 1;
+        }
+        const bool wide = vec && u < UI;  // the slot is V elements
+        const int gx = x0 + c, gy = y0 - 1 + ry;
+        const bool ok = gx <= p.nx && gy <= p.ny;
+        R *d = s + ry * L::P + L::O + c;
+        const R *g = f;
+        if (ok) g += (int64_t)nbmap(gy, p.ny, p.bc) * p.nx + nbmap(gx, p.nx, p.bc);
+        for (int k = 0; k < q; ++k, d += L::FIELD, g += n) {
+            if (ok && chunk) {
+                cp_16(d, g);
+                continue;
+            }
+            if (ok) cp_elem(d, g);
+            else *d = R(0);
+            if (wide)
+                for (int j = 1; j < V; ++j) d[j] = R(0);
         }
     }
 }
 
-// Cells [c-1, c+4] of one staged row into w[0..5].
-template <typename R> __device__ __forceinline__ void ld_row6r(const R *p, R *w)
+// Four cells (16-byte aligned) of a staged row: v; with their outer neighbours
+// w[0..5].
+template <typename R> __device__ __forceinline__ void ld4(const R *p, R *v)
 {
     if constexpr (sizeof(R) == 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(p);
-        w[1] = v.x; w[2] = v.y; w[3] = v.z; w[4] = v.w;
+        const float4 a = *reinterpret_cast<const float4 *>(p);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     } else {
         const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
-        w[1] = a.x; w[2] = a.y; w[3] = b.x; w[4] = b.y;
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
     }
-    w[0] = p[-1];
-    w[5] = p[4];
 }
 
-// gg_lap_s's neighbour sum, from the window rows up / md / dn around column k+1
-template <typename R> __device__ __forceinline__ R lap_w(const R *up, const R *md, const R *dn, int k, int stencil, R inv)
+// The rows of one field that a lane sweeps: its stencil's sum at four cells,
+// row by row.  Stencil 0: three-cell row sums, the middle pair of each four
+// shared; 9 e is taken off before the last row is added (see gg_tile.cuh).
+template <typename R, int ST> struct LapRows {
+    R a[4], b[4], e[4];  // ST 0: the row sums of the two rows above the next; ST 1: the rows themselves
+    R l, r;              // ST 1: the outer neighbours of row e
+    __device__ __forceinline__ static void sums(const R *p, R *v, R *h)
+    {
+        ld4(p, v);
+        const R x = v[0] + v[1], y = v[2] + v[3];
+        h[0] = p[-1] + x;
+        h[1] = x + v[2];
+        h[2] = v[1] + y;
+        h[3] = y + p[4];
+    }
+    // p: the staged row above the lane's first, row pitch P
+    __device__ __forceinline__ void start(const R *p, int P)
+    {
+        if (ST == 0) {
+            R t[4];
+            sums(p, t, a);
+            sums(p + P, e, b);
+        } else {
+            ld4(p, a);
+            ld4(p + P, e);
+            l = p[P - 1];
+            r = p[P + 4];
+        }
+    }
+    // dn: the staged row below the current one.  c: the current row's cells, m: their stencil sums; moves on.
+    __device__ __forceinline__ void step(const R *dn, R *c, R *m)
+    {
+        R v[4];
+        if (ST == 0) {
+            R h[4];
+            sums(dn, v, h);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c[k] = e[k];
+                m[k] = a[k] + (b[k] + h[k] - R(9) * e[k]);
+                a[k] = b[k];
+                b[k] = h[k];
+                e[k] = v[k];
+            }
+        } else {
+            ld4(dn, v);
+            const R l2 = dn[-1], r2 = dn[4];
+            const R w[6] = {l, e[0], e[1], e[2], e[3], r};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c[k] = e[k];
+                m[k] = (w[k] + w[k + 2]) + (a[k] + v[k]) - R(4) * e[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                a[k] = e[k];
+                e[k] = v[k];
+            }
+            l = l2;
+            r = r2;
+        }
+    }
+};
+
+// Four results to global memory: the first nv of them (vec: 16-byte stores).
+template <typename R> __device__ __forceinline__ void st4(R *d, const R *v, int nv, bool vec)
 {
-    R v;
-    if (stencil == 0)
-        v = up[k] + up[k + 1] + up[k + 2] + md[k] + md[k + 2] + dn[k] + dn[k + 1] + dn[k + 2] - R(8) * md[k + 1];
-    else
-        v = md[k] + md[k + 2] + up[k + 1] + dn[k + 1] - R(4) * md[k + 1];
-    return v * inv;
+    if (vec && nv >= 4) {
+        if constexpr (sizeof(R) == 4) {
+            *reinterpret_cast<float4 *>(d) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            *reinterpret_cast<double2 *>(d) = make_double2(v[0], v[1]);
+            *reinterpret_cast<double2 *>(d + 2) = make_double2(v[2], v[3]);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < nv) d[k] = v[k];
+    }
 }
 
-template <typename R>
+// PARTS warps share a field's rows.
+template <typename R, int TY, int PARTS, int ST>
 __global__ void __launch_bounds__(kAdjThreads) gg_fwd32_kernel(GgAdj p, ParamSrc ps, const R *__restrict__ eta,
                                                                R *__restrict__ out)
 {
-    using L = G32<R>;
+    using L = G32<R, TY>;
+    constexpr int RPT = TY / 4 / PARTS;  // rows a lane
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *se = reinterpret_cast<R *>(smem_raw), *sS = se + p.q * L::FIELD;
-    double mobil, grcoef, gamma;
-    int64_t step;
-    load_params(ps, mobil, grcoef, gamma, step);
-    const int ntx = p.nx / L::T, tx = blockIdx.x % ntx, ty = blockIdx.x / ntx;
-    gg_stage32(se, eta, p.q, tx, ty, p);
+    __shared__ GgConst<R> sc;
+    R *se = reinterpret_cast<R *>(smem_raw), *sG = se + p.q * L::FIELD;
+    const int ntx = (p.nx + 31) / 32, x0 = blockIdx.x % ntx * 32, y0 = blockIdx.x / ntx * TY;
+    pdl_trigger();
+    pdl_wait();
+    gg_stage32<R, TY>(se, eta, p.q, x0, y0, p, p.vin);
+    if (threadIdx.x == kAdjThreads - 1) {
+        double mobil, grcoef, gamma;
+        int64_t step;
+        load_params(ps, mobil, grcoef, gamma, step);
+        sc.set(p, mobil, grcoef, gamma);
+    }
     gg_stage_wait();
     __syncthreads();
+    const R dtm = sc.dtm, g2 = sc.g2, m2 = sc.m2, ki = sc.ki;
+    // FP64: G = 2 gamma S - 1 and dfd = e*(G + (1 - 2 gamma) e^2), two operations a
+    // field fewer; FP32 keeps S and the form whose terms cancel exactly in a grain's
+    // interior (there the separately rounded 2 gamma and 1 - 2 gamma would not)
+    constexpr bool D = sizeof(R) == 8;
     {
-        const int row = threadIdx.x / 8, c = (threadIdx.x % 8) * 4;
-        R acc[4] = {R(0), R(0), R(0), R(0)};
+        constexpr int C = TY / 8;  // cells a thread: every thread, for the serial sum over the fields
+        const int row = threadIdx.x / (L::T / C), c = threadIdx.x % (L::T / C) * C;
+        R acc[C] = {};
         for (int k = 0; k < p.q; ++k) {
-            const R *q = se + k * L::FIELD + (row + 1) * L::P + L::O + c;
+            const R *v = se + k * L::FIELD + (row + 1) * L::P + L::O + c;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += q[j] * q[j];
+            for (int j = 0; j < C; ++j) acc[j] += v[j] * v[j];
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sS[row * L::T + c + j] = acc[j];
+        for (int j = 0; j < C; ++j) sG[row * L::T + c + j] = D ? g2 * acc[j] - R(1) : acc[j];
     }
     __syncthreads();
     const int64_t n = (int64_t)p.nx * p.ny;
-    const R dtm = R(p.dt * mobil), g2 = R(2.0 * gamma), kap = R(grcoef), inv = R(1.0 / p.dxdy);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = (lane & 7) * 4, r0 = (lane >> 3) * kG32Rows;
-    const int64_t gbase = (int64_t)(ty * L::T + r0) * p.nx + tx * L::T + c0;
-    for (int f = warp; f < p.q; f += kAdjThreads / 32) {
-        const R *fs = se + f * L::FIELD + L::O + c0;
-        R w[3][6];
-        ld_row6r(fs + r0 * L::P, w[0]);
-        ld_row6r(fs + (r0 + 1) * L::P, w[1]);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = (lane & 7) * 4;
+    const int nv = p.nx - x0 - c0;  // valid cells from the lane's first on
+    for (int u = warp; u < p.q * PARTS; u += kAdjThreads / 32) {
+        const int f = u / PARTS, r0 = ((lane >> 3) + u % PARTS * 4) * RPT;
+        const R *fs = se + f * L::FIELD + r0 * L::P + L::O + c0;
+        LapRows<R, ST> w;
+        w.start(fs, L::P);
+        R *dst = out + f * n + (int64_t)(y0 + r0) * p.nx + x0 + c0;
 #pragma unroll
-        for (int i = 0; i < kG32Rows; ++i) {
-            const R *up = w[i % 3], *md = w[(i + 1) % 3];
-            R *dn = w[(i + 2) % 3];
-            ld_row6r(fs + (r0 + i + 2) * L::P, dn);
-            R o4[4];
+        for (int i = 0; i < RPT; ++i) {
+            R e[4], m[4], G[4], o[4];
+            w.step(fs + (i + 2) * L::P, e, m);
+            ld4(sG + (r0 + i) * L::T + c0, G);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const R e = md[k + 1], e2 = e * e, S = sS[(r0 + i) * L::T + c0 + k];
-                const R dfd = e * (e2 - R(1) + g2 * (S - e2));
-                o4[k] = e - dtm * (dfd - kap * lap_w(up, md, dn, k, p.stencil, inv));
+                const R e2 = e[k] * e[k], b = D ? G[k] + m2 * e2 : (e2 - R(1)) + g2 * (G[k] - e2);
+                o[k] = e[k] - dtm * (e[k] * b - ki * m[k]);
             }
-            R *dst = out + f * n + gbase + (int64_t)i * p.nx;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[k] = o4[k];
+            if (y0 + r0 + i < p.ny) st4(dst + (int64_t)i * p.nx, o, nv, p.vout);
         }
     }
 }
 
-// Input cotangents of all q fields and dL/d(L, kappa, gamma) into gparams
-// (gg_adj_kernel's arithmetic; the parameter sums are grouped differently).
-template <typename R>
-__global__ void __launch_bounds__(kAdjThreads) gg_adj32_kernel(GgAdj p, ParamSrc ps, const R *__restrict__ eta,
-                                                               const R *__restrict__ gout, R *__restrict__ gin,
-                                                               double *__restrict__ gparams)
+// Input cotangents of all q fields and dL/d(L, kappa, gamma) into gparams:
+//   b = e^2 - 1 + 2 gamma (S - e^2),  dfd_k = e*b,
+//   gin_k = g_k - dtL*(g_k*(b + 2 e^2) + 4 gamma e (P - g_k e) - kappa lap g_k).
+template <typename R, int TY, int PARTS, int ST>
+__global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? 4 : 2)
+    gg_adj32_kernel(GgAdj p, ParamSrc ps, const R *__restrict__ eta, const R *__restrict__ gout, R *__restrict__ gin,
+                    double *__restrict__ gparams)
 {
-    using L = G32<R>;
+    using L = G32<R, TY>;
+    constexpr int RPT = TY / 4 / PARTS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[kAdjThreads / 32];
+    __shared__ GgConst<R> sc;
     R *se = reinterpret_cast<R *>(smem_raw), *sg = se + p.q * L::FIELD;
-    R *sS = sg + p.q * L::FIELD, *sP = sS + L::T * L::T;
-    double mobil, grcoef, gamma;
-    int64_t step;
-    load_params(ps, mobil, grcoef, gamma, step);
-    const int ntx = p.nx / L::T, tx = blockIdx.x % ntx, ty = blockIdx.x / ntx;
-    gg_stage32(se, eta, p.q, tx, ty, p);
-    gg_stage32(sg, gout, p.q, tx, ty, p);
+    R *sS = sg + p.q * L::FIELD, *sP = sS + TY * L::T;
+    const int ntx = (p.nx + 31) / 32, x0 = blockIdx.x % ntx * 32, y0 = blockIdx.x / ntx * TY;
+    pdl_trigger();
+    pdl_wait();
+    gg_stage32<R, TY>(se, eta, p.q, x0, y0, p, p.vin);
+    gg_stage32<R, TY>(sg, gout, p.q, x0, y0, p, p.vg);
+    if (threadIdx.x == kAdjThreads - 1) {
+        double mobil, grcoef, gamma;
+        int64_t step;
+        load_params(ps, mobil, grcoef, gamma, step);
+        sc.set(p, mobil, grcoef, gamma);
+    }
     gg_stage_wait();
     __syncthreads();
     {
-        const int row = threadIdx.x / 8, c = (threadIdx.x % 8) * 4;
-        R S[4] = {R(0), R(0), R(0), R(0)}, P[4] = {R(0), R(0), R(0), R(0)};
+        constexpr int C = TY / 8;
+        const int row = threadIdx.x / (L::T / C), c = threadIdx.x % (L::T / C) * C;
+        R S[C] = {}, P[C] = {};
         for (int k = 0; k < p.q; ++k) {
             const int o = k * L::FIELD + (row + 1) * L::P + L::O + c;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < C; ++j) {
                 const R e = se[o + j];
                 S[j] += e * e;
                 P[j] += sg[o + j] * e;
             }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < C; ++j) {
             sS[row * L::T + c + j] = S[j];
             sP[row * L::T + c + j] = P[j];
         }
     }
     __syncthreads();
     const int64_t n = (int64_t)p.nx * p.ny;
-    const R dt = R(p.dt), dtm = R(p.dt * mobil), gm = R(gamma), kap = R(grcoef), inv = R(1.0 / p.dxdy);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = (lane & 7) * 4, r0 = (lane >> 3) * kG32Rows;
-    const int64_t gbase = (int64_t)(ty * L::T + r0) * p.nx + tx * L::T + c0;
-    R gl = R(0), gkap = R(0), ggam = R(0);
-    for (int f = warp; f < p.q; f += kAdjThreads / 32) {
-        const R *fe = se + f * L::FIELD + L::O + c0, *fg = sg + f * L::FIELD + L::O + c0;
-        R we[3][6], wg[3][6];
-        ld_row6r(fe + r0 * L::P, we[0]);
-        ld_row6r(fe + (r0 + 1) * L::P, we[1]);
-        ld_row6r(fg + r0 * L::P, wg[0]);
-        ld_row6r(fg + (r0 + 1) * L::P, wg[1]);
-#pragma unroll
-        for (int i = 0; i < kG32Rows; ++i) {
-            const R *eu = we[i % 3], *em = we[(i + 1) % 3], *gu = wg[i % 3], *gmr = wg[(i + 1) % 3];
-            R *ed = we[(i + 2) % 3], *gd = wg[(i + 2) % 3];
-            ld_row6r(fe + (r0 + i + 2) * L::P, ed);
-            ld_row6r(fg + (r0 + i + 2) * L::P, gd);
-            R o4[4];
+    const R dtm = sc.dtm, g2 = sc.g2, g4 = sc.g4, ki = sc.ki;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = (lane & 7) * 4;
+    const int nv = p.nx - x0 - c0;
+    R gl = R(0), gkap = R(0), ggam = R(0);  // sums of g*(dfd - kappa lap e), g*(stencil sum of e), g*e*(S - e^2)
+    for (int u = warp; u < p.q * PARTS; u += kAdjThreads / 32) {
+        const int f = u / PARTS, r0 = ((lane >> 3) + u % PARTS * 4) * RPT;
+        const int o0 = f * L::FIELD + r0 * L::P + L::O + c0;
+        LapRows<R, ST> we, wg;
+        we.start(se + o0, L::P);
+        wg.start(sg + o0, L::P);
+        R *dst = gin + f * n + (int64_t)(y0 + r0) * p.nx + x0 + c0;
+#pragma unroll 1  // (unrolled, the next rows' loads are hoisted and spill)
+        for (int i = 0; i < RPT; ++i) {
+            R e[4], g[4], me[4], mg[4], S[4], P[4], o[4];
+            we.step(se + o0 + (i + 2) * L::P, e, me);
+            wg.step(sg + o0 + (i + 2) * L::P, g, mg);
+            ld4(sS + (r0 + i) * L::T + c0, S);
+            ld4(sP + (r0 + i) * L::T + c0, P);
+            const bool row = y0 + r0 + i < p.ny;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int so = (r0 + i) * L::T + c0 + k;
-                const R S = sS[so], P = sP[so];
-                const R e = em[k + 1], e2 = e * e, gk = gmr[k + 1];
-                const R jac = R(3) * e2 - R(1) + R(2) * gm * (S - e2);  // d dfd_k / d eta_k
-                o4[k] = gk - dtm * (gk * jac + R(4) * gm * e * (P - gk * e)) +
-                        dtm * kap * lap_w(gu, gmr, gd, k, p.stencil, inv);
-                const R lap = lap_w(eu, em, ed, k, p.stencil, inv);
-                const R dfd = e * (e2 - R(1) + R(2) * gm * (S - e2));
-                gl += gk * (-dt) * (dfd - kap * lap);
-                gkap += gk * dtm * lap;
-                ggam += gk * (-dtm) * R(2) * e * (S - e2);
+                const R e2 = e[k] * e[k], s1 = S[k] - e2, b = (e2 - R(1)) + g2 * s1, x = g[k] * e[k];
+                o[k] = g[k] - dtm * (g[k] * (b + R(2) * e2) + (g4 * e[k]) * (P[k] - x) - ki * mg[k]);
+                if (row && k < nv) {
+                    gl += g[k] * (e[k] * b - ki * me[k]);
+                    gkap += g[k] * me[k];
+                    ggam += x * s1;
+                }
             }
-            R *dst = gin + f * n + gbase + (int64_t)i * p.nx;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dst[k] = o4[k];
+            if (row) st4(dst + (int64_t)i * p.nx, o, nv, p.vout);
         }
     }
-    const double a = block_sum(gl, red);
-    const double b = block_sum(gkap, red);
-    const double c = block_sum(ggam, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(&gparams[0], a);
-        atomicAdd(&gparams[1], b);
-        atomicAdd(&gparams[2], c);
-    }
-}
-
-// The 32x32 periodic path applies (and its staging fits in shared memory)?
-template <typename R> bool gg_use32(const amps_params *p, int sums)
-{
-    return p->bc == AMPS_BC_PERIODIC && p->nx % 32 == 0 && p->ny % 32 == 0 &&
-           G32<R>::smem(sums == 2 ? 2 * p->nfields : p->nfields, sums) <= (size_t)kMaxAdjSmem;
+    // (the staging is over 3 * 256 values)
+    block_sums<kAdjThreads>(se, gl, gkap, ggam, sc.sl, sc.sk, sc.sg, gparams);
 }
 
 // ------------------------------------------------------------- launches ----
@@ -796,35 +843,81 @@ template <typename R, int TY> constexpr size_t kob_adj_smem()
 // 32x16 tiles, or 32x8 where that leaves fewer than two CTAs per SM.
 bool small_tiles(int nx, int ny) { return (int64_t)((nx + 31) / 32) * ((ny + 15) / 16) < 2 * 152; }
 
-// Largest dynamic shared memory of any launch (grain growth with 32 fields
-// in double: 2 * 32 * 340 * 8 = 174 KB).
 template <typename R> cudaError_t kob_prepare()
 {
     const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(kob_adj_kernel<R, kTX, 16>, attr, (int)kob_adj_smem<R, 16>());
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kob_adj_kernel<R, kTX, 8>, attr, (int)kob_adj_smem<R, 8>());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_fwd_kernel<R>, attr, (int)(32 * GReg::N * sizeof(R)));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_adj_kernel<R>, attr, (int)(2 * 32 * GReg::N * sizeof(R)));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_fwd32_kernel<R>, attr, kMaxAdjSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_adj32_kernel<R>, attr, kMaxAdjSmem);
     return e;
 }
 
-KobAdj kob_args(const amps_params *p)
+// Calls fn(TY, PARTS, ST as integral constants) for a grain-growth launch
+// (kernel: `sets` staged states, `sums` sum tiles): 16 rows, or 8 where those
+// of all fields do not fit or would leave SMs without a tile; a field to 1, 2
+// or 4 warps by the fields.
+template <typename R, typename F> auto gg_dispatch(int nx, int ny, int q, int stencil, int sets, int sums, F fn)
 {
-    KobAdj k;
+    using std::integral_constant;
+    auto st = [&](auto ty, auto parts) {
+        return stencil == 0 ? fn(ty, parts, integral_constant<int, 0>()) : fn(ty, parts, integral_constant<int, 1>());
+    };
+    const integral_constant<int, 1> one;
+    const integral_constant<int, 2> two;
+    if (G32<R, 16>::smem(sets * q, sums) > (size_t)kMaxAdjSmem ||
+        (int64_t)((nx + 31) / 32) * ((ny + 15) / 16) < 152) {
+        const integral_constant<int, 8> ty;
+        return q > 4 ? st(ty, one) : st(ty, two);
+    }
+    const integral_constant<int, 16> ty;
+    if (q >= 8) return st(ty, one);
+    if (q >= 4) return st(ty, two);
+    return st(ty, integral_constant<int, 4>());
+}
+
+template <typename R> cudaError_t gg_prepare_adj()
+{
+    const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaSuccess;
+    for (int stencil = 0; stencil < 2; ++stencil)
+        for (int q : {1, 4, 8})
+            for (int side : {8, 4096})  // few tiles, many
+                gg_dispatch<R>(side, side, q, stencil, 1, 1, [&](auto ty, auto parts, auto st) {
+                    const auto fwd = gg_fwd32_kernel<R, ty(), parts(), st()>;
+                    const auto adj = gg_adj32_kernel<R, ty(), parts(), st()>;
+                    if (e == cudaSuccess) e = cudaFuncSetAttribute(fwd, attr, kMaxAdjSmem);
+                    if (e == cudaSuccess) e = cudaFuncSetAttribute(adj, attr, kMaxAdjSmem);
+                });
+    return e;
+}
+
+template <typename R> KobAdj<R> kob_args(const amps_params *p)
+{
+    KobAdj<R> k;
     k.nx = p->nx; k.ny = p->ny; k.bc = p->bc;
-    k.dx = p->dx; k.dy = p->dy; k.dxdy = p->dx * p->dy; k.dt = p->dt; k.tau = p->tau;
-    k.aniso = p->aniso; k.theta0 = p->theta0; k.alpha = p->alpha; k.gama = p->gama;
-    k.teq = p->teq; k.pi = p->pi; k.noise = p->noise; k.seed = p->seed;
+    const bool even = p->aniso >= 2 && p->aniso <= 16 && p->aniso == 2 * floor(p->aniso / 2);
+    k.mode = even ? (int)p->aniso : 0;
+    k.noisy = p->noise != 0.0;
+    k.seed = p->seed;
+    k.aniso_d = p->aniso;
+    k.hx = R(0.5 / p->dx); k.hy = R(0.5 / p->dy); k.aniso = R(p->aniso); k.theta0 = R(p->theta0);
+    k.c0 = R(cos(p->aniso * p->theta0)); k.s0 = R(sin(p->aniso * p->theta0));
+    k.dtt = R(p->dt / p->tau); k.inv = R(1.0 / (p->dx * p->dy)); k.m = R(p->alpha / p->pi); k.gama = R(p->gama);
+    k.teq = R(p->teq); k.noise = R(p->noise); k.dt = R(p->dt); k.dtinv = R(p->dt * k.inv);
     return k;
 }
 
-GgAdj gg_args(const amps_params *p)
+// whether 16-byte accesses to rows of `ptr` are aligned
+template <typename R> bool vec_ok(const amps_params *p, const void *ptr)
+{
+    return p->nx % (16 / (int)sizeof(R)) == 0 && (uintptr_t)ptr % 16 == 0;
+}
+
+template <typename R> GgAdj gg_args(const amps_params *p, const void *in, const void *gout, const void *out)
 {
     GgAdj g;
+    g.vin = vec_ok<R>(p, in); g.vg = vec_ok<R>(p, gout); g.vout = vec_ok<R>(p, out);
     g.nx = p->nx; g.ny = p->ny; g.bc = p->bc; g.q = p->nfields; g.stencil = p->stencil;
-    g.dxdy = p->dx * p->dy; g.dt = p->dt;
+    g.inv = 1.0 / (p->dx * p->dy); g.dt = p->dt;
     return g;
 }
 
@@ -857,6 +950,24 @@ int64_t state_elems(const amps_params *p)
     return (int64_t)p->nx * p->ny * (p->model == AMPS_KOBAYASHI ? 2 : p->nfields);
 }
 
+// A launch that may start while the stream's previous grid drains: every
+// kernel here waits for it (griddepcontrol.wait) before its first global read.
+template <typename K, typename... Args>
+void launch2(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);  // (the callers read cudaGetLastError)
+}
+
 template <typename R>
 void launch_forward(const amps_params *p, const ParamSrc &ps, const void *in, void *out, cudaStream_t s)
 {
@@ -864,20 +975,19 @@ void launch_forward(const amps_params *p, const ParamSrc &ps, const void *in, vo
     if (p->model == AMPS_KOBAYASHI) {
         if (small_tiles(nx, ny)) {
             const dim3 grid((nx + kTX - 1) / kTX, (ny + 7) / 8);
-            kob_fwd_kernel<R, kTX, 8><<<grid, kAdjThreads, kob_fwd_smem<R, 8>(), s>>>(kob_args(p), ps, (const R *)in,
-                                                                                      (R *)out);
+            launch2(kob_fwd_kernel<R, kTX, 8>, grid, kob_fwd_threads<8>(), kob_fwd_smem<R, 8>(), s, kob_args<R>(p), ps,
+                    (const R *)in, (R *)out);
         } else {
             const dim3 grid((nx + kTX - 1) / kTX, (ny + 15) / 16);
-            kob_fwd_kernel<R, kTX, 16><<<grid, kAdjThreads, kob_fwd_smem<R, 16>(), s>>>(kob_args(p), ps,
-                                                                                        (const R *)in, (R *)out);
+            launch2(kob_fwd_kernel<R, kTX, 16>, grid, kob_fwd_threads<16>(), kob_fwd_smem<R, 16>(), s, kob_args<R>(p),
+                    ps, (const R *)in, (R *)out);
         }
-    } else if (gg_use32<R>(p, 1)) {
-        gg_fwd32_kernel<R><<<(nx / 32) * (ny / 32), kAdjThreads, G32<R>::smem(p->nfields, 1), s>>>(
-            gg_args(p), ps, (const R *)in, (R *)out);
     } else {
-        const dim3 grid((nx + kGX - 1) / kGX, (ny + kGY - 1) / kGY);
-        gg_fwd_kernel<R><<<grid, kAdjThreads, (size_t)p->nfields * GReg::N * sizeof(R), s>>>(gg_args(p), ps,
-                                                                                            (const R *)in, (R *)out);
+        const GgAdj g = gg_args<R>(p, in, nullptr, out);
+        gg_dispatch<R>(nx, ny, p->nfields, p->stencil, 1, 1, [&](auto ty, auto parts, auto st) {
+            launch2(gg_fwd32_kernel<R, ty(), parts(), st()>, dim3((nx + 31) / 32 * ((ny + ty() - 1) / ty())), kAdjThreads,
+                    G32<R, ty()>::smem(p->nfields, 1), s, g, ps, (const R *)in, (R *)out);
+        });
     }
 }
 
@@ -889,20 +999,19 @@ void launch_adjoint(const amps_params *p, const ParamSrc &ps, const void *in, co
     if (p->model == AMPS_KOBAYASHI) {
         if (small_tiles(nx, ny)) {
             const dim3 grid((nx + kTX - 1) / kTX, (ny + 7) / 8);
-            kob_adj_kernel<R, kTX, 8><<<grid, kAdjThreads, kob_adj_smem<R, 8>(), s>>>(
-                kob_args(p), ps, (const R *)in, (const R *)gout, (R *)gin, gparams);
+            launch2(kob_adj_kernel<R, kTX, 8>, grid, kob_adj_threads<8>(), kob_adj_smem<R, 8>(), s, kob_args<R>(p), ps,
+                    (const R *)in, (const R *)gout, (R *)gin, gparams);
         } else {
             const dim3 grid((nx + kTX - 1) / kTX, (ny + 15) / 16);
-            kob_adj_kernel<R, kTX, 16><<<grid, kAdjThreads, kob_adj_smem<R, 16>(), s>>>(
-                kob_args(p), ps, (const R *)in, (const R *)gout, (R *)gin, gparams);
+            launch2(kob_adj_kernel<R, kTX, 16>, grid, kob_adj_threads<16>(), kob_adj_smem<R, 16>(), s, kob_args<R>(p), ps,
+                    (const R *)in, (const R *)gout, (R *)gin, gparams);
         }
-    } else if (gg_use32<R>(p, 2)) {
-        gg_adj32_kernel<R><<<(nx / 32) * (ny / 32), kAdjThreads, G32<R>::smem(2 * p->nfields, 2), s>>>(
-            gg_args(p), ps, (const R *)in, (const R *)gout, (R *)gin, gparams);
     } else {
-        const dim3 grid((nx + kGX - 1) / kGX, (ny + kGY - 1) / kGY);
-        gg_adj_kernel<R><<<grid, kAdjThreads, 2 * (size_t)p->nfields * GReg::N * sizeof(R), s>>>(
-            gg_args(p), ps, (const R *)in, (const R *)gout, (R *)gin, gparams);
+        const GgAdj g = gg_args<R>(p, in, gout, gin);
+        gg_dispatch<R>(nx, ny, p->nfields, p->stencil, 2, 2, [&](auto ty, auto parts, auto st) {
+            launch2(gg_adj32_kernel<R, ty(), parts(), st()>, dim3((nx + 31) / 32 * ((ny + ty() - 1) / ty())), kAdjThreads,
+                    G32<R, ty()>::smem(2 * p->nfields, 2), s, g, ps, (const R *)in, (const R *)gout, (R *)gin, gparams);
+        });
     }
 }
 
@@ -910,7 +1019,10 @@ cudaError_t prepare(int dtype)
 {
     static cudaError_t done[2] = {cudaErrorNotReady, cudaErrorNotReady};
     const int k = dtype == AMPS_F64 ? 0 : 1;
-    if (done[k] != cudaSuccess) done[k] = k == 0 ? kob_prepare<double>() : kob_prepare<float>();
+    if (done[k] != cudaSuccess) {
+        done[k] = k == 0 ? kob_prepare<double>() : kob_prepare<float>();
+        if (done[k] == cudaSuccess) done[k] = k == 0 ? gg_prepare_adj<double>() : gg_prepare_adj<float>();
+    }
     return done[k];
 }
 
