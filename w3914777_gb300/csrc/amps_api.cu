@@ -224,6 +224,8 @@ static Phys make_phys(const amps_params &p)
         k[SN_INV] = ph.inv_dxdy; k[SN_B] = ph.B; k[SN_A2] = 2.0 * ph.A; k[SN_HCM] = 0.5 * ph.coefm;
         k[SN_DVOL] = ph.dvol; k[SN_DVAP] = ph.dvap; k[SN_DSUR] = ph.dsur; k[SN_DGRB] = ph.dgrb; k[SN_DT] = ph.dt;
         k[SN_B12] = 12.0 * ph.B; k[SN_DTL] = ph.dt * ph.coefl; k[SN_HCK] = 0.5 * ph.coefk;
+        k[SN_HCMI] = k[SN_HCM] * k[SN_INV]; k[SN_HCKI] = k[SN_HCK] * k[SN_INV]; k[SN_DTI] = ph.dt * k[SN_INV];
+        k[SN_DVD] = ph.dvol - ph.dvap;
     }
     for (int i = 0; i < KCONST_MAX; ++i) ph.kf[i] = (float)ph.kd[i];
     return ph;

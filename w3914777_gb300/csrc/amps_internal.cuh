@@ -59,8 +59,10 @@ enum KConst {
     // aniso*theta0, 2dx, 2dy
     KB_HX, KB_HY, KB_ANISO, KB_THETA0, KB_EPSB, KB_DELTA, KB_ED, KB_M, KB_GAMA, KB_TEQ, KB_NOISE, KB_DTT,
     KB_KAPPA, KB_DT, KB_INV, KB_MODE, KB_C0, KB_S0, KB_DX2, KB_DY2,
-    // sintering: 1/dxdy, B, 2A, 0.5*coefm, dvol, dvap, dsur, dgrb, dt, 12B, dt*coefl, 0.5*coefk
+    // sintering: 1/dxdy, B, 2A, 0.5*coefm, dvol, dvap, dsur, dgrb, dt, 12B, dt*coefl, 0.5*coefk,
+    // 0.5*coefm/dxdy, 0.5*coefk/dxdy, dt/dxdy, dvol - dvap
     SN_INV = 0, SN_B, SN_A2, SN_HCM, SN_DVOL, SN_DVAP, SN_DSUR, SN_DGRB, SN_DT, SN_B12, SN_DTL, SN_HCK,
+    SN_HCMI, SN_HCKI, SN_DTI, SN_DVD,
     // grain growth's FP64 tiles: 2*gamma, 1 - 2*gamma, kappa/(dx*dy), dt*L
     GG_G2 = 0, GG_M2, GG_KI, GG_DTM,
     KCONST_MAX = 24
@@ -375,12 +377,13 @@ __device__ __forceinline__ void load_neighbour_tiers(const StepArgs &a, int tx, 
 // an interior 8-cell row segment (16-byte vector loads) or one halo cell --
 // whose coordinates, tier and offsets are computed once; the field loop then
 // only adds the field stride, issuing a batch of loads before any store.
+// tid: the thread's index among the NT that stage (the last overload: threadIdx.x).
 // SKIP32: the FP32-owned slots already hold their values (copied by this
 // same thread: stage_tile_async32 gives every thread the same slots); only
 // the others are loaded and converted.
 template <typename CT, int T, int R, bool SKIP32 = false, bool NC = true, int NT = kThreads>
 __device__ __forceinline__ void stage_tile(const StepArgs &a, CT *sm, const uint8_t *nt, int tx, int ty, int f0,
-                                           int nfs)
+                                           int nfs, int tid)
 {
     using S = Stage<CT, T, R>;
     constexpr int SEG = T / 8;
@@ -395,7 +398,7 @@ __device__ __forceinline__ void stage_tile(const StepArgs &a, CT *sm, const uint
     int64_t goff[SLOTS];
 #pragma unroll
     for (int q = 0; q < SLOTS; ++q) {
-        const int u = threadIdx.x + q * NT;
+        const int u = tid + q * NT;
         kind[q] = 0; tier[q] = 0; soff[q] = 0; goff[q] = 0;
         if (u < UI) {
             const int sg = u % SEG, r = u / SEG;
@@ -512,27 +515,60 @@ __device__ __forceinline__ void stage_tile(const StepArgs &a, CT *sm, const uint
     }
 }
 
+template <typename CT, int T, int R, bool SKIP32 = false, bool NC = true, int NT = kThreads>
+__device__ __forceinline__ void stage_tile(const StepArgs &a, CT *sm, const uint8_t *nt, int tx, int ty, int f0,
+                                           int nfs)
+{
+    stage_tile<CT, T, R, SKIP32, NC, NT>(a, sm, nt, tx, ty, f0, nfs, (int)threadIdx.x);
+}
+
 // Rows per CTA of the band kernels (a tile of a non-monitor step split into
 // T / kBandRows row bands, one CTA each).
 constexpr int kBandRows = 8;
 
-// Rows [ly0, ly0 + H) x columns [-R, T + R) (tile-local) of fields
+// Rows [ly0, ly0 + H) x columns [-R, T + R) (tile-local, R <= 2) of fields
 // [f0, f0 + nfs) of tile (tx, ty), each cell read at its owner tile's input
-// tier (nt: load_neighbour_tiers) and converted to CT, into dst[f][H][T + 2R]
-// (a row band of a tile, for the band kernels).
-template <typename CT, int T, int R>
-__device__ __forceinline__ void stage_band(const StepArgs &a, CT *dst, const uint8_t *nt, int tx, int ty, int ly0,
+// tier (nt: load_neighbour_tiers) and converted to double, into
+// dst[f][H][T + 4], column 0 of the tile at column 2 (a row band of a tile, for
+// the band kernels of NT threads).  FP64 cells come by asynchronous copies, 16
+// bytes in the interior, every field in flight at once: stage_band_wait before
+// the caller's barrier.
+template <int T, int R, int NT = kThreads>
+__device__ __forceinline__ void stage_band(const StepArgs &a, double *dst, const uint8_t *nt, int tx, int ty, int ly0,
                                            int H, int f0, int nfs)
 {
-    constexpr int W = T + 2 * R;
+    constexpr int P = T + 4, SL = T / 2 + 2 * R;  // slots a row: interior pairs, then halo cells
     const int x0 = tx * T, y0 = ty * T;
-    for (int u = threadIdx.x; u < H * W; u += kThreads) {
-        const int ly = ly0 + u / W, lx = u % W - R;
+    for (int u = threadIdx.x; u < H * SL; u += NT) {
+        const int r = u / SL, k = u % SL, ly = ly0 + r;
+        const bool pair = k < T / 2;
+        const int h = k - T / 2, lx = pair ? 2 * k : (h < R ? h - R : T + h - R);
         const int tier = nt[(ly < 0 ? 0 : (ly < T ? 3 : 6)) + (lx < 0 ? 0 : (lx < T ? 1 : 2))];
         const int64_t off = (int64_t)bc_map(y0 + ly, a.ny, a.bc) * a.px + bc_map(x0 + lx, a.nx, a.bc);
+        double *d = dst + r * P + 2 + lx;
+        if (tier == TIER_FP64) {
+            const double *src = (const double *)a.in[TIER_FP64] + (int64_t)f0 * a.n + off;
+            for (int f = 0; f < nfs; ++f, d += H * P, src += a.n) {
+                if (pair)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(src) : "memory");
+                else
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d)), "l"(src) : "memory");
+            }
+        } else {
 #pragma unroll 4
-        for (int f = 0; f < nfs; ++f) dst[f * H * W + u] = load_tier<CT>(a, tier, (int64_t)(f0 + f) * a.n + off);
+            for (int f = 0; f < nfs; ++f) {
+                const int64_t i = (int64_t)(f0 + f) * a.n + off;
+                d[f * H * P] = load_tier<double>(a, tier, i);
+                if (pair) d[f * H * P + 1] = load_tier<double>(a, tier, i + 1);
+            }
+        }
     }
+}
+
+__device__ __forceinline__ void stage_band_wait()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // Stage fields [f0, f0 + nfs) of a tile whose whole 3x3 neighbourhood holds FP32

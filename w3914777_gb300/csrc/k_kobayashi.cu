@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __gri
         const int x0 = tx * T, y0 = ty * T;
         load_neighbour_tiers(a, tx, ty, ntier);
         __syncthreads();  // (also: the previous item's reads of the staging)
-        stage_band<double, T, 2>(a, sp, ntier, tx, ty, ly0 - 2, br + 4, 0, 2);
+        stage_band<T, 2>(a, sp, ntier, tx, ty, ly0 - 2, br + 4, 0, 2);
+        stage_band_wait();
         __syncthreads();
         // with zero flux an out-of-domain ring cell takes the values of the
         // cell it mirrors, which lies in the same band
