@@ -495,9 +495,7 @@ static int reclassify_resting(amps_handle *h)
                                     h->stream));
             // every tile to the high tier for the first period
             h->all_fp64 = p.model == AMPS_GRAINGROWTH && p.high_tier == TIER_FP64 && h->sched_n == 0 && p.thr_hi <= 1e300;
-            std::vector<double> big(h->ntiles, 1e300);
-            CK(h, cudaMemcpyAsync(h->d_metric, big.data(), sizeof(double) * h->ntiles, cudaMemcpyHostToDevice, h->stream));
-            CK(h, cudaStreamSynchronize(h->stream));
+            CK(h, fill_doubles(h->d_metric, h->ntiles, 1e300, h->stream));
         } else {
             h->all_fp64 = false;
             CK(h, monitor_state(g, 1, p.monitor_samples, p.monitor_field, h->d_metric, nullptr, 0, h->d_flags, h->stream));
@@ -543,8 +541,8 @@ static int static_tiers(amps_handle *h)
     return AMPS_OK;
 }
 
-// Write the staged [nf][n] doubles (d_stage) as the current state.
-static int commit_stage(amps_handle *h)
+// Write [nf][n] doubles or floats on the device (src) as the current state.
+static int commit_fields(amps_handle *h, const void *src, int src_f32)
 {
     if (h->p.mode == AMPS_END2END_MIX) {
         // resting state lives at the high tier until the monitor has looked at it
@@ -552,7 +550,7 @@ static int commit_stage(amps_handle *h)
         CK(h, cudaMemsetAsync(h->d_tier_prev, h->p.high_tier, h->ntiles, h->stream));
         h->transition = false;
         Grid g = grid_view(h, h->parity, h->d_tier_cur);
-        CK(h, scatter_fields(g, h->d_stage, 0, h->stream));
+        CK(h, scatter_fields(g, src, src_f32, h->stream));
         int r = reclassify_resting(h);
         if (r) return r;
     } else {
@@ -560,10 +558,12 @@ static int commit_stage(amps_handle *h)
         if (r) return r;
         h->transition = false;
         Grid g = grid_view(h, h->parity, h->d_tier_cur);
-        CK(h, scatter_fields(g, h->d_stage, 0, h->stream));
+        CK(h, scatter_fields(g, src, src_f32, h->stream));
     }
     return AMPS_OK;
 }
+
+static int commit_stage(amps_handle *h) { return commit_fields(h, h->d_stage, 0); }
 
 extern "C" int amps_init(amps_handle *h, int kind)
 {
@@ -583,6 +583,16 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
 {
     if (!h || !src || (dtype != AMPS_F64 && dtype != AMPS_F32) || f0 < 0 || f0 + nfs > h->nf)
         return AMPS_ERR_INVALID;
+    if (on_device && nfs == h->nf) {
+        // the whole state from device memory: stored straight from the caller's
+        // array, read before the call returns (but for spatial-monitor runs,
+        // which queue the read on the handle's stream)
+        const int r = commit_fields(h, src, dtype == AMPS_F32);
+        if (r) return r;
+        if (h->p.mode != AMPS_END2END_MIX || h->p.monitor != AMPS_MONITOR_SPA || dtype == AMPS_F32)
+            CK(h, cudaStreamSynchronize(h->stream));
+        return AMPS_OK;
+    }
     // every field must be in the stage: fetch the others first
     Grid live = grid_view(h, h->parity, live_tiers(h));
     if (nfs < h->nf) CK(h, gather_fields(live, h->d_stage, 0, 0, h->nf, h->stream));

@@ -91,6 +91,7 @@ struct Grid {
 // Row-major [nf][ny][nx] double/float <-> tiered storage (pitch px, field stride fs).
 cudaError_t scatter_fields(const Grid &g, const void *src, int src_f32, cudaStream_t s);
 cudaError_t gather_fields(const Grid &g, void *dst, int dst_f32, int f0, int nfs, cudaStream_t s);
+cudaError_t fill_doubles(double *p, int n, double v, cudaStream_t s);
 // Monitor at time 0 (or after a set_field): metric and temporal snapshot from the state.
 // diff != 0 (kind 2): metric = max |state - snap| over the samples instead of the range.
 cudaError_t monitor_state(const Grid &g, int kind, int samples, int mfield, double *metric, double *snap,
@@ -111,7 +112,7 @@ struct ClassifyArgs {
     int64_t *step_base;
     int advance;                // steps to add to *step_base (one period, or 0)
     int stat_steps;             // steps the current counts ran for (tile-step stats)
-    int *order;                 // optional: launch order of the fused grain-growth step
+    int *order;                 // launch order of the fused grain-growth step
     int bc;                     // boundary map of the tile neighbourhood (for order)
     // optional tier schedule: the k-th classification takes its tier map from
     // sched[min(k, sched_n - 1)] instead of the metric (*sched_i = k, advanced here)

@@ -19,21 +19,6 @@ __device__ __forceinline__ int64_t store_index(const Grid &g, int f, int x, int 
     return (int64_t)f * g.fs + (int64_t)y * g.px + x;
 }
 
-__global__ void scatter_kernel(Grid g, const void *src, int src_f32)
-{
-    const int64_t total = (int64_t)g.nf * g.n;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = k % g.n;
-        const int x = (int)(c % g.nx), y = (int)(c / g.nx);
-        const double v = src_f32 ? (double)((const float *)src)[k] : ((const double *)src)[k];
-        const int t = tier_of(g, x, y);
-        const int64_t q = store_index(g, (int)(k / g.n), x, y);
-        if (t == TIER_FP64) ((double *)g.store[2])[q] = v;
-        else if (t == TIER_FP32) ((float *)g.store[1])[q] = (float)v;
-        else ((__half *)g.store[0])[q] = __float2half_rn((float)v);
-    }
-}
-
 // c: index of the cell in the row-major domain array
 __device__ __forceinline__ double read_cell(const Grid &g, int f, int64_t c)
 {
@@ -45,31 +30,151 @@ __device__ __forceinline__ double read_cell(const Grid &g, int f, int64_t c)
     return (double)__half2float(((const __half *)g.store[0])[k]);
 }
 
-__global__ void gather_kernel(Grid g, void *dst, int dst_f32, int f0, int nfs)
+// Row-major [nf][ny][nx] arrays <-> the tiered storage, a CTA per tile and
+// kXferFields fields: the tile's tier is one uniform branch, a thread moves
+// four cells of a row with 16-byte accesses (V: rows of the array are 16-byte
+// aligned) and no address takes a division per cell.  Bound by HBM: 2048^2 Q=8, cold,
+// FP64 in 157 us (and an 80 us copy before it) with a division per cell and 8-byte
+// accesses, 77 now; FP32 out 157, 40 now.
+constexpr int kXferFields = 4;
+
+template <typename S> __device__ __forceinline__ void put4(S *d, const double v[4], int n, bool vec)
 {
-    const int64_t total = (int64_t)nfs * g.n;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const double v = read_cell(g, f0 + (int)(k / g.n), k % g.n);
-        if (dst_f32) ((float *)dst)[k] = (float)v;
-        else ((double *)dst)[k] = v;
+    if (vec && n == 4) {
+        if constexpr (sizeof(S) == 8) {
+            reinterpret_cast<double2 *>(d)[0] = make_double2(v[0], v[1]);
+            reinterpret_cast<double2 *>(d)[1] = make_double2(v[2], v[3]);
+        } else {
+            *reinterpret_cast<float4 *>(d) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k < n) d[k] = (S)v[k];
+}
+
+// The storage of a ragged grid's edge tile reaches past the domain: zeros there.
+template <int T, typename S>
+__global__ void __launch_bounds__(256) scatter_kernel(Grid g, const S *__restrict__ src, bool vec)
+{
+    constexpr int TPT = T * T / 4, PER = 256 / TPT;
+    const int tile = blockIdx.x, l = threadIdx.x % TPT;
+    const int x = tile % g.ntx * T + l % (T / 4) * 4, y = tile / g.ntx * T + l / (T / 4);
+    if (x >= g.nx || y >= g.ny) return;
+    const int t = g.tier[tile], n = g.nx - x < 4 ? g.nx - x : 4;
+#pragma unroll
+    for (int j = threadIdx.x / TPT; j < kXferFields; j += PER) {
+        const int f = blockIdx.y * kXferFields + j;
+        if (f >= g.nf) break;
+        const S *p = src + (int64_t)f * g.n + (int64_t)y * g.nx + x;
+        const int64_t o = (int64_t)f * g.fs + (int64_t)y * g.px + x;
+        S v[4] = {S(0), S(0), S(0), S(0)};
+        if (vec && n == 4) {
+            if constexpr (sizeof(S) == 8) {
+                const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+                v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+            } else {
+                const float4 a = *reinterpret_cast<const float4 *>(p);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k < n) v[k] = p[k];
+        }
+        if (t == TIER_FP64) {
+            double2 *d = reinterpret_cast<double2 *>((double *)g.store[2] + o);
+            d[0] = make_double2((double)v[0], (double)v[1]);
+            d[1] = make_double2((double)v[2], (double)v[3]);
+        } else if (t == TIER_FP32) {
+            *reinterpret_cast<float4 *>((float *)g.store[1] + o) =
+                make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+        } else {
+            const __half2 a = __floats2half2_rn((float)v[0], (float)v[1]), b = __floats2half2_rn((float)v[2], (float)v[3]);
+            uint2 u;
+            u.x = *reinterpret_cast<const unsigned *>(&a);
+            u.y = *reinterpret_cast<const unsigned *>(&b);
+            *reinterpret_cast<uint2 *>((__half *)g.store[0] + o) = u;
+        }
     }
 }
 
-static int grid_for(int64_t total)
+template <int T, typename S>
+__global__ void __launch_bounds__(256) gather_kernel(Grid g, S *dst, int f0, int nfs, bool vec)
 {
-    int64_t b = (total + 255) / 256;
-    return (int)(b > 152 * 16 ? 152 * 16 : (b < 1 ? 1 : b));
+    constexpr int TPT = T * T / 4, PER = 256 / TPT;
+    const int tile = blockIdx.x, l = threadIdx.x % TPT;
+    const int x = tile % g.ntx * T + l % (T / 4) * 4, y = tile / g.ntx * T + l / (T / 4);
+    if (x >= g.nx || y >= g.ny) return;
+    const int t = g.tier[tile], n = g.nx - x < 4 ? g.nx - x : 4;
+#pragma unroll
+    for (int j = threadIdx.x / TPT; j < kXferFields; j += PER) {
+        const int f = blockIdx.y * kXferFields + j;
+        if (f >= nfs) break;
+        const int64_t o = (int64_t)(f0 + f) * g.fs + (int64_t)y * g.px + x;
+        S *p = dst + (int64_t)f * g.n + (int64_t)y * g.nx + x;
+        if (sizeof(S) == 4 && t != TIER_FP64) {  // float to float: no FP64 conversion
+            float v[4];
+            load4f(g, t, o, v);
+            if (vec && n == 4) {
+                *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < n) p[k] = (S)v[k];
+            }
+            continue;
+        }
+        double v[4];
+        load4d(g, t, o, v);
+        put4(p, v, n, vec);
+    }
+}
+
+template <typename S> static bool rows_aligned(const Grid &g, const void *p)
+{
+    return g.nx % (16 / (int)sizeof(S)) == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+}
+
+template <typename S> static void scatter_t(const Grid &g, const void *src, cudaStream_t s)
+{
+    const dim3 grid(g.ntx * g.nty, (g.nf + kXferFields - 1) / kXferFields);
+    const bool vec = rows_aligned<S>(g, src);
+    if (g.tile == 32) scatter_kernel<32, S><<<grid, 256, 0, s>>>(g, (const S *)src, vec);
+    else scatter_kernel<16, S><<<grid, 256, 0, s>>>(g, (const S *)src, vec);
+}
+
+template <typename S> static void gather_t(const Grid &g, void *dst, int f0, int nfs, cudaStream_t s)
+{
+    const dim3 grid(g.ntx * g.nty, (nfs + kXferFields - 1) / kXferFields);
+    const bool vec = rows_aligned<S>(g, dst);
+    if (g.tile == 32) gather_kernel<32, S><<<grid, 256, 0, s>>>(g, (S *)dst, f0, nfs, vec);
+    else gather_kernel<16, S><<<grid, 256, 0, s>>>(g, (S *)dst, f0, nfs, vec);
 }
 
 cudaError_t scatter_fields(const Grid &g, const void *src, int src_f32, cudaStream_t s)
 {
-    scatter_kernel<<<grid_for((int64_t)g.nf * g.n), 256, 0, s>>>(g, src, src_f32);
+    if (src_f32) scatter_t<float>(g, src, s);
+    else scatter_t<double>(g, src, s);
     return cudaGetLastError();
 }
 
 cudaError_t gather_fields(const Grid &g, void *dst, int dst_f32, int f0, int nfs, cudaStream_t s)
 {
-    gather_kernel<<<grid_for((int64_t)nfs * g.n), 256, 0, s>>>(g, dst, dst_f32, f0, nfs);
+    if (dst_f32) gather_t<float>(g, dst, f0, nfs, s);
+    else gather_t<double>(g, dst, f0, nfs, s);
+    return cudaGetLastError();
+}
+
+__global__ void fill_kernel(double *p, int n, double v)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
+}
+
+cudaError_t fill_doubles(double *p, int n, double v, cudaStream_t s)
+{
+    fill_kernel<<<(n + 1023) / 1024 < 152 ? (n + 1023) / 1024 : 152, 256, 0, s>>>(p, n, v);
     return cudaGetLastError();
 }
 
@@ -271,69 +376,24 @@ __device__ void lists_from_tiers(const uint8_t *tier, int ntiles, int *lists, in
     if (threadIdx.x < 3) counts[threadIdx.x] = (int)((base >> (21 * threadIdx.x)) & AMPS_MAX_TILES);
 }
 
-// Launch order of the fused grain-growth step: first the tiles that take
-// its slow paths -- FP64 or half tiles, and FP32 tiles with a neighbour
-// (after the boundary map) at another tier, which stage their neighbourhood
-// with conversions -- then the all-FP32 neighbourhoods, each group in tile
-// order.  Slow tiles then run in the first wave, where their extra time is
-// absorbed, instead of straggling at the end of the step.  Scheduling only:
-// every tile is computed by exactly one CTA either way.
-__device__ void order_slow_first(const ClassifyArgs &c, const uint8_t *tier, unsigned long long *ws)
-{
-    __shared__ unsigned long long base;
-    __shared__ int nslow;
-    const int ntiles = c.ntx * c.nty;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();  // also: this block's tier_cur writes are visible to it
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int t0 = 0; t0 < ntiles; t0 += blockDim.x) {
-            const int t = t0 + threadIdx.x;
-            bool slow = false;
-            if (t < ntiles) {
-                const int x = t % c.ntx, y = t / c.ntx;
-                for (int dy = -1; dy <= 1; ++dy)
-                    for (int dx = -1; dx <= 1; ++dx) {
-                        int yy = y + dy, xx = x + dx;
-                        if (c.bc == 0) {
-                            yy = yy < 0 ? yy + c.nty : (yy >= c.nty ? yy - c.nty : yy);
-                            xx = xx < 0 ? xx + c.ntx : (xx >= c.ntx ? xx - c.ntx : xx);
-                        } else {
-                            yy = yy < 0 ? 0 : (yy >= c.nty ? c.nty - 1 : yy);
-                            xx = xx < 0 ? 0 : (xx >= c.ntx ? c.ntx - 1 : xx);
-                        }
-                        slow |= tier[yy * c.ntx + xx] != TIER_FP32;
-                    }
-            }
-            // pass 0 places the slow tiles, pass 1 (after nslow of them) the others
-            const bool mine = t < ntiles && slow == (pass == 0);
-            const unsigned long long inc = block_scan((unsigned long long)mine, ws);
-            const unsigned long long b = base;
-            if (mine) c.order[(pass ? nslow : 0) + (int)(b + inc - 1)] = t;
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1) base = b + inc;
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            if (pass == 0) nslow = (int)base;
-            base = 0;
-        }
-        __syncthreads();
-    }
-}
-
-// lists_from_tiers and order_slow_first in one pass, for maps of at most one
-// tile per thread: one scan of two packed counters -- the tier ranks, and
-// the slow (low 32 bits) / all-FP32 (high 32 bits) ranks of the launch
-// order.  Same lists, counts and order as the two routines.
+// The per-tier tile lists and counts, and the launch order of the fused
+// grain-growth step: first the tiles that take its slow paths -- FP64 or half
+// tiles, and FP32 tiles with a neighbour (after the boundary map) at another
+// tier, which stage their neighbourhood with conversions -- then the all-FP32
+// neighbourhoods, each group in tile order.  Slow tiles then run in the first
+// wave, where their extra time is absorbed, instead of straggling at the end
+// of the step.  Scheduling only: every tile is computed by exactly one CTA
+// either way.  A thread ranks a tile, or in larger maps a run of consecutive
+// tiles, so one scan of two
+// packed counters -- the tier ranks, and the slow (low 32 bits) / all-FP32
+// (high 32 bits) ranks -- serves maps of any size: a 4096-tile map's
+// classification, cold, 27 us with a scan per 1024 tiles and list, 19 now.
 __device__ void lists_and_order(const ClassifyArgs &c, const uint8_t *tier, unsigned long long *ws)
 {
     const int ntiles = c.ntx * c.nty;
-    const int t = threadIdx.x;
-    int k = -1;
-    bool slow = false;
-    if (t < ntiles) {
-        k = tier[t];
+    auto slow_at = [&](int t) {
         const int x = t % c.ntx, y = t / c.ntx;
+        bool slow = false;
         for (int dy = -1; dy <= 1; ++dy)
             for (int dx = -1; dx <= 1; ++dx) {
                 int yy = y + dy, xx = x + dx;
@@ -346,17 +406,45 @@ __device__ void lists_and_order(const ClassifyArgs &c, const uint8_t *tier, unsi
                 }
                 slow |= tier[yy * c.ntx + xx] != TIER_FP32;
             }
+        return slow;
+    };
+    if (ntiles <= (int)blockDim.x) {  // a tile a thread
+        const int t = threadIdx.x, k = t < ntiles ? tier[t] : -1;
+        const bool slow = k >= 0 && slow_at(t);
+        const unsigned long long ma = k >= 0 ? (1ull << (21 * k)) : 0ull;
+        const unsigned long long mb = k >= 0 ? (slow ? 1ull : (1ull << 32)) : 0ull;
+        unsigned long long a = ma, b = mb, ta, tb;
+        block_scan2(a, b, ws, &ta, &tb);
+        if (k >= 0) {
+            const unsigned long long ea = a - ma, eb = b - mb;
+            c.lists[k * ntiles + (int)((ea >> (21 * k)) & AMPS_MAX_TILES)] = t;
+            c.order[slow ? (int)(eb & 0xFFFFFFFFull) : (int)(tb & 0xFFFFFFFFull) + (int)(eb >> 32)] = t;
+        }
+        if (t < 3) c.counts[t] = (int)((ta >> (21 * t)) & AMPS_MAX_TILES);
+        return;
     }
-    const unsigned long long ma = k >= 0 ? (1ull << (21 * k)) : 0ull;
-    const unsigned long long mb = k >= 0 ? (slow ? 1ull : (1ull << 32)) : 0ull;
+    const int per = (ntiles + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int t0 = min((int)threadIdx.x * per, ntiles), t1 = min(t0 + per, ntiles);
+    unsigned long long ma = 0, mb = 0, slows = 0;  // slows: bit i, tile t0 + i (the first 64 of the run)
+    for (int t = t0; t < t1; ++t) {
+        const bool slow = slow_at(t);
+        if (t - t0 < 64) slows |= (unsigned long long)slow << (t - t0);
+        ma += 1ull << (21 * tier[t]);
+        mb += slow ? 1ull : (1ull << 32);
+    }
     unsigned long long a = ma, b = mb, ta, tb;
     block_scan2(a, b, ws, &ta, &tb);
-    if (k >= 0) {
-        const unsigned long long ea = a - ma, eb = b - mb;
+    unsigned long long ea = a - ma, eb = b - mb;
+    const int nslow = (int)(tb & 0xFFFFFFFFull);
+    for (int t = t0; t < t1; ++t) {
+        const int k = tier[t];
+        const bool slow = t - t0 < 64 ? (slows >> (t - t0) & 1ull) != 0ull : slow_at(t);
         c.lists[k * ntiles + (int)((ea >> (21 * k)) & AMPS_MAX_TILES)] = t;
-        c.order[slow ? (int)(eb & 0xFFFFFFFFull) : (int)(tb & 0xFFFFFFFFull) + (int)(eb >> 32)] = t;
+        c.order[slow ? (int)(eb & 0xFFFFFFFFull) : nslow + (int)(eb >> 32)] = t;
+        ea += 1ull << (21 * k);
+        eb += slow ? 1ull : (1ull << 32);
     }
-    if (t < 3) c.counts[t] = (int)((ta >> (21 * t)) & AMPS_MAX_TILES);
+    if (threadIdx.x < 3) c.counts[threadIdx.x] = (int)((ta >> (21 * threadIdx.x)) & AMPS_MAX_TILES);
 }
 
 // Tier maps of up to this many tiles are also kept in the classifying CTA's
@@ -405,12 +493,7 @@ __device__ void classify_body(const ClassifyArgs &c)
     atomicAdd(&dem, nd);
     __syncthreads();
     const uint8_t *tier = in_smem ? s_tier : c.tier_cur;
-    if (c.order && ntiles <= (int)blockDim.x) {
-        lists_and_order(c, tier, ws);
-    } else {
-        lists_from_tiers(tier, ntiles, c.lists, c.counts, ws);
-        if (c.order) order_slow_first(c, tier, ws);
-    }
+    lists_and_order(c, tier, ws);
     if (threadIdx.x == 0) {
         c.stats[4] += prom;
         c.stats[5] += dem;
