@@ -249,7 +249,7 @@ __device__ __forceinline__ void gg_tile_lo_rows(const StepArgs &a, const float *
 // fused operation; the division by dx*dy is div_known; pow(eta, 3) is the
 // correctly rounded cube (cube_rn), within an ulp of any library's pow.  About
 // 27 FP64 operations a cell and field at Q = 2 in place of ~137 with pow and
-// the general division: 32 us a step in place of 103 on the reference's 512^2
+// the general division: 30 us a step in place of 103 on the reference's 512^2
 // two-field adaptive run, nearly all of whose 16^2 tiles hold a moving boundary.
 template <int T> struct Stage64 {
     static constexpr int O = 2, P = T + 2 * O;  // interior at column 2: 16-byte aligned rows
@@ -491,6 +491,9 @@ __device__ __forceinline__ void gg_tile_fp64(const StepArgs &a, float *smf, cons
         const int rot = 2 * (tile & 3);
         if (T == 32 && hb == 16 && a.nf % 8 == 0) gg_band64<T, REF, T == 32 ? 8 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
         else if (T == 32 && hb == 16) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        // (one row a lane keeps all eight warps of a two-field 16^2 tile busy:
+        // 32.4 -> 30.1 us a step of the reference's 512^2 adaptive run)
+        else if (REF && a.nf <= 2) gg_band64<T, REF, REF ? 1 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
         else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot);
         __syncthreads();  // the next band overwrites the staging; the monitor reads the stored tile
     }
