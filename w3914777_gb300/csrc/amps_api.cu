@@ -1289,7 +1289,7 @@ extern "C" int amps_get_kernel_times(amps_handle *h, double *ms, int64_t *launch
 // the members and replayed.
 struct amps_ensemble {
     std::vector<amps_handle *> m;
-    int T = 0, cad = 0, maxnf = 0;
+    int T = 0, cad = 0;
     bool ref = false, mixed = false;
     cudaStream_t stream = nullptr, capture = nullptr;
     // members launched together: same occupancy class, at most kEnsCap
@@ -1377,21 +1377,22 @@ extern "C" int amps_ensemble_create(amps_handle *const *members, int count, amps
     e->cad = h0->p.cadence;
     e->mixed = h0->mixed;
     e->ref = h0->p.ref_order != 0;
-    for (int i = 0; i < count; ++i) e->maxnf = std::max(e->maxnf, members[i]->nf);
-    // groups: members with more fields first; a group closes where the
-    // occupancy its largest member's staging allows would change, or at kEnsCap
+    // groups: members with the larger staging first, whose size a group's launches
+    // take (16^2 tiles: 16 fields stage more than 17, gg_fp64_band); a group closes
+    // where the occupancy that its first member's staging allows would change, or at kEnsCap
+    auto staging = [&](int i) { return gg_ens_smem_bytes(e->T, members[i]->nf); };
     std::vector<int> order(count);
     for (int i = 0; i < count; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return members[a]->nf > members[b]->nf; });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return staging(a) > staging(b); });
     std::vector<ClassifyArgs> cls(count);
     for (int i = 0; i < count; ++i) cls[i] = classify_args(members[i], e->cad, e->cad);
-    cudaError_t ce = gg_prepare_ens(e->T, e->ref, gg_ens_smem_bytes(e->T, e->maxnf));
+    cudaError_t ce = gg_prepare_ens(e->T, e->ref, staging(order[0]));
     std::map<int, int> occ;  // field count -> CTAs an SM
     for (int i = 0; ce == cudaSuccess && i < count; ++i) {
         const int nf = members[order[i]]->nf;
         if (!occ.count(nf)) {
             int bps = 0;
-            ce = gg_ens_occupancy(e->T, e->ref, gg_ens_smem_bytes(e->T, nf), &bps);
+            ce = gg_ens_occupancy(e->T, e->ref, staging(order[i]), &bps);
             if (ce == cudaSuccess && bps < 1) ce = cudaErrorInvalidConfiguration;
             occ[nf] = bps;
         }
@@ -1401,7 +1402,7 @@ extern "C" int amps_ensemble_create(amps_handle *const *members, int count, amps
         if (e->groups.empty() || (int)e->groups.back().members.size() == kEnsCap ||
             occ[e->m[e->groups.back().members[0]]->nf] != occ[h->nf]) {
             e->groups.emplace_back();
-            e->groups.back().smem = gg_ens_smem_bytes(e->T, h->nf);
+            e->groups.back().smem = staging(order[i]);
             e->groups.back().first.push_back(0);
         }
         auto &g = e->groups.back();

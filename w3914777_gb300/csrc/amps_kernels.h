@@ -65,7 +65,7 @@ struct EnsLaunch {
     StepArgs m[kEnsCap];
 };
 static_assert(sizeof(EnsLaunch) <= 32764, "kernel parameter space");
-size_t gg_ens_smem_bytes(int tile, int max_nf);
+size_t gg_ens_smem_bytes(int tile, int nf);
 // sets the kernels' dynamic shared-memory limit to max_smem
 cudaError_t gg_prepare_ens(int tile, bool ref, size_t max_smem);
 cudaError_t gg_ens_occupancy(int tile, bool ref, size_t smem, int *blocks_per_sm);

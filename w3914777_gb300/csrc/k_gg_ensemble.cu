@@ -183,8 +183,8 @@ cudaError_t gg_launch_ens_pair(const EnsLaunch &L, size_t smem, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// staging for a group's member with the most fields
-size_t gg_ens_smem_bytes(int tile, int max_nf) { return gg_smem_bytes(tile, max_nf); }
+// staging of a member (not monotonic in its fields: gg_fp64_band)
+size_t gg_ens_smem_bytes(int tile, int nf) { return gg_smem_bytes(tile, nf); }
 
 #define AMPS_GGE_DISPATCH(MACRO) \
     do {                         \
