@@ -205,6 +205,8 @@ AMPS_API int amps_init(amps_handle *h, int kind);
  * double [ny][nx] each).  Needs no GPU. */
 AMPS_API int amps_init_host(const amps_params *p, int kind, double *const *fields);
 /* Set / get one field.  on_device: 0 = host pointer, 1 = device pointer.
+ * The source has been read when a set returns (but inside a capture of the
+ * handle's stream), so it may be reused or freed at once.
  * amps_get_field replaces data_sychro_aftercomputation +
  * purelow2high_aftercomputing (snowflake/tools.h:108-174). */
 AMPS_API int amps_set_field(amps_handle *h, int field, const void *src, int dtype, int on_device);

@@ -71,6 +71,7 @@ struct amps_handle {
     // private stream on which a handle working on the default stream (which
     // cannot be captured) captures its period graphs; replayed on the default stream
     cudaStream_t cap = nullptr;
+    cudaEvent_t read = nullptr;  // set_impl: the caller's array has been read
 
     int64_t step = 0;
     int64_t launches = 0;  // kernels enqueued by the run loop (graph replays add their graph's count)
@@ -263,6 +264,7 @@ static void free_all(amps_handle *h)
     if (h->h_pinned) cudaFreeHost(h->h_pinned);
     if (h->own) cudaStreamDestroy(h->own);
     if (h->cap) cudaStreamDestroy(h->cap);
+    if (h->read) cudaEventDestroy(h->read);
 }
 
 extern "C" int amps_create(const amps_params *p, amps_handle **out)
@@ -342,6 +344,8 @@ extern "C" int amps_create(const amps_params *p, amps_handle **out)
 #undef ALLOC
     if (cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking) != cudaSuccess)
         return fail(AMPS_ERR_CUDA, "stream");
+    if (cudaEventCreateWithFlags(&h->read, cudaEventDisableTiming) != cudaSuccess)
+        return fail(AMPS_ERR_CUDA, "event");
 
     h->stream = h->own;
     cudaMemsetAsync(h->d_stats, 0, sizeof(unsigned long long) * 8, h->stream);
@@ -542,7 +546,8 @@ static int static_tiers(amps_handle *h)
 }
 
 // Write [nf][n] doubles or floats on the device (src) as the current state.
-static int commit_fields(amps_handle *h, const void *src, int src_f32)
+// read: an event recorded behind the last operation that reads src.
+static int commit_fields(amps_handle *h, const void *src, int src_f32, cudaEvent_t read = nullptr)
 {
     if (h->p.mode == AMPS_END2END_MIX) {
         // resting state lives at the high tier until the monitor has looked at it
@@ -551,6 +556,7 @@ static int commit_fields(amps_handle *h, const void *src, int src_f32)
         h->transition = false;
         Grid g = grid_view(h, h->parity, h->d_tier_cur);
         CK(h, scatter_fields(g, src, src_f32, h->stream));
+        if (read) CK(h, cudaEventRecord(read, h->stream));
         int r = reclassify_resting(h);
         if (r) return r;
     } else {
@@ -559,6 +565,7 @@ static int commit_fields(amps_handle *h, const void *src, int src_f32)
         h->transition = false;
         Grid g = grid_view(h, h->parity, h->d_tier_cur);
         CK(h, scatter_fields(g, src, src_f32, h->stream));
+        if (read) CK(h, cudaEventRecord(read, h->stream));
     }
     return AMPS_OK;
 }
@@ -583,14 +590,19 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
 {
     if (!h || !src || (dtype != AMPS_F64 && dtype != AMPS_F32) || f0 < 0 || f0 + nfs > h->nf)
         return AMPS_ERR_INVALID;
+    // The caller's array has been read when this returns, in every mode: it may be
+    // refilled, or freed and its memory handed out again, at once.  (The state of a
+    // spatial-monitor run may be set inside a capture of the handle's stream, which
+    // cannot be waited for.)
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (dtype == AMPS_F64 && h->p.mode == AMPS_END2END_MIX && h->p.monitor == AMPS_MONITOR_SPA)
+        CK(h, cudaStreamIsCapturing(h->stream, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (on_device && nfs == h->nf) {
-        // the whole state from device memory: stored straight from the caller's
-        // array, read before the call returns (but for spatial-monitor runs,
-        // which queue the read on the handle's stream)
-        const int r = commit_fields(h, src, dtype == AMPS_F32);
+        // the whole state from device memory: stored straight from the caller's array
+        const int r = commit_fields(h, src, dtype == AMPS_F32, capturing ? nullptr : h->read);
         if (r) return r;
-        if (h->p.mode != AMPS_END2END_MIX || h->p.monitor != AMPS_MONITOR_SPA || dtype == AMPS_F32)
-            CK(h, cudaStreamSynchronize(h->stream));
+        if (!capturing) CK(h, cudaEventSynchronize(h->read));
         return AMPS_OK;
     }
     // every field must be in the stage: fetch the others first
@@ -600,6 +612,7 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
     double *dst = h->d_stage + (int64_t)f0 * h->n;
     if (dtype == AMPS_F64) {
         CK(h, cudaMemcpyAsync(dst, src, cnt * 8, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
+        if (!capturing) CK(h, cudaEventRecord(h->read, h->stream));
     } else {
         // float input (a set-up path, not the time loop): widened to double
         // on the host, through the pinned buffer
@@ -612,8 +625,12 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
             for (size_t i = 0; i < cnt; ++i) h->h_pinned[i] = ((const float *)src)[i];
         }
         CK(h, cudaMemcpyAsync(dst, h->h_pinned, cnt * 8, cudaMemcpyHostToDevice, h->stream));
+        return commit_stage(h);
     }
-    return commit_stage(h);
+    const int r = commit_stage(h);
+    if (r) return r;
+    if (!capturing) CK(h, cudaEventSynchronize(h->read));
+    return AMPS_OK;
 }
 
 extern "C" int amps_set_field(amps_handle *h, int field, const void *src, int dtype, int on_device)
