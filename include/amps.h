@@ -206,7 +206,10 @@ AMPS_API int amps_init(amps_handle *h, int kind);
 AMPS_API int amps_init_host(const amps_params *p, int kind, double *const *fields);
 /* Set / get one field.  on_device: 0 = host pointer, 1 = device pointer.
  * The source has been read when a set returns (but inside a capture of the
- * handle's stream), so it may be reused or freed at once.
+ * handle's stream), so it may be reused or freed at once.  A float device
+ * source is read after the work queued on the legacy default stream, a double
+ * one in the order of the handle's stream only: work on another stream that
+ * produces it has to be waited for, or ordered before that stream.
  * amps_get_field replaces data_sychro_aftercomputation +
  * purelow2high_aftercomputing (snowflake/tools.h:108-174). */
 AMPS_API int amps_set_field(amps_handle *h, int field, const void *src, int dtype, int on_device);

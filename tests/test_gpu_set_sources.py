@@ -59,3 +59,22 @@ def test_source_may_be_overwritten_on_return(run, field, source, dtype):
         torch.cuda.synchronize()
         got = s.fields()
     assert np.array_equal(got if field is None else got[field], want.numpy())
+
+
+@pytest.mark.parametrize("run", sorted(RUNS))
+@pytest.mark.parametrize("field", [None, 1])
+def test_float_device_source_follows_the_default_stream(run, field):
+    """A float array that work on the default stream is still to write when the
+    state is set, with no synchronisation of the caller's."""
+    shape = (3, NY, NX) if field is None else (NY, NX)
+    want = _values(shape, 6)
+    made = want.float().cuda()
+    src = torch.full(shape, 0.5, dtype=torch.float32, device="cuda")
+    with _sim(run) as s:
+        s.synchronize()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)
+        src.copy_(made)
+        _set(s, field, src.data_ptr(), w.F32, 1)
+        got = s.fields()
+    assert np.array_equal(got if field is None else got[field], want.numpy())

@@ -247,7 +247,9 @@ class Simulation:
         assert a.shape == (self.nf,) + self.shape
         self._ck(lib().amps_set_fields(self.h, a.ctypes.data, F64, 0), "amps_set_fields")
 
-    # device pointers (e.g. torch tensors' data_ptr()) -- no host round trip
+    # device pointers (e.g. torch tensors' data_ptr()) -- no host round trip; the
+    # array is read by the time a set returns, a double one in the order of the
+    # handle's stream only (synchronize what produces it first)
     def set_fields_device(self, ptr, dtype=F64):
         self._ck(lib().amps_set_fields(self.h, ctypes.c_void_p(ptr), dtype, 1), "amps_set_fields")
 

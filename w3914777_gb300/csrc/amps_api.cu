@@ -599,7 +599,13 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
         CK(h, cudaStreamIsCapturing(h->stream, &cs));
     const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (on_device && nfs == h->nf) {
-        // the whole state from device memory: stored straight from the caller's array
+        // the whole state from device memory: stored straight from the caller's array.
+        // A float array is read after what is queued on the legacy default stream (a
+        // caller need not wait there for it to be complete)
+        if (dtype == AMPS_F32 && h->stream) {
+            CK(h, cudaEventRecord(h->read, cudaStreamLegacy));
+            CK(h, cudaStreamWaitEvent(h->stream, h->read, 0));
+        }
         const int r = commit_fields(h, src, dtype == AMPS_F32, capturing ? nullptr : h->read);
         if (r) return r;
         if (!capturing) CK(h, cudaEventSynchronize(h->read));
