@@ -78,3 +78,43 @@ def test_float_device_source_follows_the_default_stream(run, field):
         _set(s, field, src.data_ptr(), w.F32, 1)
         got = s.fields()
     assert np.array_equal(got if field is None else got[field], want.numpy())
+
+
+def _managed(nbytes):
+    """Managed memory, from the driver."""
+    cuda = ctypes.CDLL("libcuda.so.1")
+    p = ctypes.c_uint64()
+    assert cuda.cuMemAllocManaged(ctypes.byref(p), ctypes.c_size_t(nbytes), 1) == 0
+    return cuda, p
+
+
+@pytest.mark.parametrize("run", ["plain", "spa", "rate"])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("source", ["bytes", "managed", "inside"])
+def test_device_sources_that_a_kernel_cannot_or_may_read_in_place(run, dtype, source):
+    """A device array at an odd address, and managed memory, are copied; one
+    that ends with its allocation is read in place."""
+    tt, code, npt = (torch.float64, w.F64, np.float64) if dtype == "f64" else (torch.float32, w.F32, np.float32)
+    want = _values((3, NY, NX), 7)
+    host = np.ascontiguousarray(want.numpy().astype(npt))
+    cuda = p = None
+    if source == "managed":
+        torch.cuda.synchronize()
+        cuda, p = _managed(host.nbytes)
+        ctypes.memmove(p.value, host.ctypes.data, host.nbytes)
+        ptr = p.value
+    elif source == "bytes":
+        buf = torch.zeros(host.nbytes + 16, dtype=torch.uint8, device="cuda")
+        buf[2:2 + host.nbytes].copy_(torch.from_numpy(host.view(np.uint8).reshape(-1)))
+        ptr = buf.data_ptr() + 2
+    else:
+        buf = torch.zeros(host.size + 64, dtype=tt, device="cuda")
+        buf[64:].copy_(torch.from_numpy(host).reshape(-1))
+        ptr = buf[64:].data_ptr()
+    torch.cuda.synchronize()
+    with _sim(run) as s:
+        _set(s, None, ptr, code, 1)
+        got = s.fields()
+    if p is not None:
+        cuda.cuMemFree_v2(p)
+    assert np.array_equal(got, want.numpy())

@@ -586,6 +586,35 @@ extern "C" int amps_init(amps_handle *h, int kind)
     return commit_stage(h);
 }
 
+// Whether a kernel may read [src, src + bytes) itself: aligned elements in an
+// allocation of the current device that reaches that far.  Other pointers
+// (another device's or managed memory, an odd address, too short an array) take
+// the copy, which stages what it can read and refuses what it cannot.
+static bool readable_in_place(const void *src, size_t bytes, size_t elem)
+{
+    if (reinterpret_cast<uintptr_t>(src) % elem) return false;
+    using Range = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
+    static const Range range = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess
+                   ? reinterpret_cast<Range>(p)
+                   : nullptr;
+    }();
+    cudaPointerAttributes at;
+    int dev = -1;
+    if (!range || cudaPointerGetAttributes(&at, src) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(src);
+    return at.type == cudaMemoryTypeDevice && at.device == dev && range(&base, &size, p) == CUDA_SUCCESS &&
+           p - base <= size && bytes <= size - (p - base);
+}
+
 static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype, int on_device)
 {
     if (!h || !src || (dtype != AMPS_F64 && dtype != AMPS_F32) || f0 < 0 || f0 + nfs > h->nf)
@@ -598,7 +627,8 @@ static int set_impl(amps_handle *h, int f0, int nfs, const void *src, int dtype,
     if (dtype == AMPS_F64 && h->p.mode == AMPS_END2END_MIX && h->p.monitor == AMPS_MONITOR_SPA)
         CK(h, cudaStreamIsCapturing(h->stream, &cs));
     const bool capturing = cs != cudaStreamCaptureStatusNone;
-    if (on_device && nfs == h->nf) {
+    if (const size_t elem = dtype == AMPS_F64 ? 8 : 4;
+        on_device && nfs == h->nf && readable_in_place(src, elem * nfs * h->n, elem)) {
         // the whole state from device memory: stored straight from the caller's array.
         // A float array is read after what is queued on the legacy default stream (a
         // caller need not wait there for it to be complete)
