@@ -417,8 +417,9 @@ __device__ __forceinline__ void sint_tile_lo32(const StepArgs &a, unsigned char 
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            // (where every eta is 0 or 1 the sums of squares and cubes are equal)
-            const bool zero = bin[k] && w[k] + w[k + 2] + dn[k] + up[k] == 4.f * w[k + 1] && w[k + 1] == s2[k];
+            // (where every eta is 0 or 1 the sums of squares and cubes are equal;
+            // x*x == x holds for +infinity too, which the sums then show)
+            const bool zero = bin[k] && w[k + 1] < INFINITY && w[k] + w[k + 2] + dn[k] + up[k] == 4.f * w[k + 1] && w[k + 1] == s2[k];
             mu[o + k] = zero ? 0.0 : sint_mu<double>(C + k, SC::P, Ec + k, SE::FIELD, np, ph);
         }
     }
