@@ -177,21 +177,21 @@ template <typename R> __device__ __forceinline__ void kob_angle(const KobAdj<R> 
     }
 }
 
-// s += v for a sum held as s + c: the rounding error of every addition is kept
-// in c (Knuth's exact two-sum), so the sum of a few floats carries twice their
-// precision without touching the FP64 pipe.
-__device__ __forceinline__ void two_sum(float &s, float &c, float v)
+// s += v exactly: returns the rounding error of the sum (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float &s, float v)
 {
-    const float t = s + v, b = t - s;
-    c += (s - (t - b)) + (v - b);
+    const float t = s + v, b = t - s, e = (s - (t - b)) + (v - b);
     s = t;
+    return e;
 }
 
 // The block's sums of three values a thread, each scaled and added into out[k].
 // FP64 addition is what costs (a warp's takes 16 cycles of an SM's pipe): the
 // threads' values meet in shared memory, three warps fold one value each (NT/32 a
-// lane, in two-float arithmetic), and only their trees are FP64.  buf: 3 * NT
-// values of shared memory, free once every thread of the block's NT is here.
+// lane, floats as s + e + f with every rounding error kept: more than FP64's 53
+// bits without its pipe), and only their trees are FP64.  A sum that leaves the
+// floats' range makes e NaN: folded again in FP64.  buf: 3 * NT values of shared
+// memory, free once every thread of the block's NT is here.
 template <int NT, typename R>
 __device__ __forceinline__ void block_sums(R *buf, R a, R b, R c, double sa, double sb, double sc, double *out)
 {
@@ -205,10 +205,15 @@ __device__ __forceinline__ void block_sums(R *buf, R a, R b, R c, double sa, dou
     const R *p = buf + w * NT + lane;
     double d;
     if constexpr (sizeof(R) == 4) {
-        float s = p[0], e = 0.f;
+        float s = p[0], e = 0.f, f = 0.f;
 #pragma unroll
-        for (int k = 1; k < NT / 32; ++k) two_sum(s, e, p[32 * k]);
-        d = (double)s + (double)e;
+        for (int k = 1; k < NT / 32; ++k) f += two_sum(e, two_sum(s, p[32 * k]));
+        d = (double)s + ((double)e + (double)f);
+        if (!(fabsf(e) < INFINITY)) {
+            d = p[0];
+#pragma unroll 1
+            for (int k = 1; k < NT / 32; ++k) d += (double)p[32 * k];
+        }
     } else {
         d = p[0];
 #pragma unroll
@@ -495,7 +500,8 @@ __global__ void __launch_bounds__(kob_adj_threads<TY>())
         gin[n + g] = gT + p.dtinv * lt + p.dtt * mu * ph * (R(1) - ph) * dm;
         gk += gT * d;
     }
-    block_sums<NT>(sphi, gd, gk, ge, 1.0, 1.0, 1.0, gparams);  // (the staging is over 3 * NT values)
+    static_assert(R3::N + 7 * R2::N + 2 * R1::N >= 3 * NT, "room of the parameter sums");
+    block_sums<NT>(sphi, gd, gk, ge, 1.0, 1.0, 1.0, gparams);
 }
 
 // --------------------------------------------------------- grain growth ----
@@ -824,7 +830,8 @@ __global__ void __launch_bounds__(kAdjThreads, sizeof(R) == 4 ? 4 : 2)
             if (row) st4(dst + (int64_t)i * p.nx, o, nv, p.vout);
         }
     }
-    // (the staging is over 3 * 256 values)
+    // (the staging and the sum tiles behind it, no longer read, hold 3 * kAdjThreads values for any q)
+    static_assert(2 * L::FIELD + 2 * TY * L::T >= 3 * kAdjThreads, "room of the parameter sums");
     block_sums<kAdjThreads>(se, gl, gkap, ggam, sc.sl, sc.sk, sc.sg, gparams);
 }
 
