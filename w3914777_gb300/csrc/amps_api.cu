@@ -809,6 +809,8 @@ static int launch_step(amps_handle *h, int step_off, bool monitor_now)
     }
     // half + FP32 in use: one launch covers both (profiled as index 3)
     const bool lo_fused = h->used[TIER_HALF] && h->used[TIER_FP32];
+    // no finite range reaches the threshold of the FP64 tier
+    const bool few64 = h->mixed && p.monitor == AMPS_MONITOR_SPA && p.thr_hi >= 1e300 && h->sched_n == 0;
     for (int t = 2; t >= 0; --t) {
         if (!h->used[t] || (lo_fused && t == TIER_HALF)) continue;
         const bool fused = lo_fused && t == TIER_FP32;
@@ -824,7 +826,7 @@ static int launch_step(amps_handle *h, int step_off, bool monitor_now)
         const bool after64 = h->used[TIER_FP64] && !h->profiling;
         if (fused) e = p.model == AMPS_KOBAYASHI ? kob_launch_lo(h->T, a, h->ntiles, st, after64)
                                                  : sint_launch_lo(h->T, p.mu_lap_fp64 != 0, a, h->ntiles, st, after64);
-        else if (p.model == AMPS_KOBAYASHI) e = kob_launch(h->T, t, ref, a, h->ntiles, st, !h->profiling);
+        else if (p.model == AMPS_KOBAYASHI) e = kob_launch(h->T, t, ref, a, h->ntiles, st, !h->profiling, few64);
         else e = sint_launch(h->T, t, ref, p.mu_lap_fp64 != 0, a, h->ntiles, st, !h->profiling);
         if (e != cudaSuccess) FAIL(h, AMPS_ERR_CUDA, "step kernel launch: %s", cudaGetErrorString(e));
         ++h->launches;

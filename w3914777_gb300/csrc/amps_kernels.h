@@ -7,8 +7,10 @@ namespace amps {
 // tm (nullable): tensor map of the step's FP32 input, used when a.tma_stage.
 cudaError_t gg_launch(int tile, bool ref, const StepArgs &a, int grid, cudaStream_t s,
                       const CUtensorMap *tm = nullptr);
-// pdl: launched programmatically after the stream's previous grid (the kernel waits for it first)
-cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl = false);
+// pdl: launched programmatically after the stream's previous grid (the kernel waits for it first);
+// few: FP64 tiles are not expected (the launch is sized for none, and right for any number)
+cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl = false,
+                       bool few = false);
 cudaError_t sint_launch(int tile, int tier, bool ref, bool mu64, const StepArgs &a, int grid, cudaStream_t s,
                         bool pdl = false);
 size_t gg_smem_bytes(int tile, int nf);

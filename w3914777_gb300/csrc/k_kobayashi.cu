@@ -367,6 +367,16 @@ __global__ void __launch_bounds__(kob_threads<T, TIER>()) kob_step_kernel(StepAr
     kob_tile<T, TIER, REF, kob_threads<T, TIER>(), true, true, POLY>(a, smraw, red, ntier, a.list[blockIdx.x]);
 }
 
+// Rows of a band: the most that still give the tiles `per_sm` CTAs an SM
+// (a band recomputes phase A on two extra rows: 1.5, 1.25, 1.13 times the
+// tile's rows for bands of 4, 8 and 16).
+__host__ __device__ __forceinline__ int kob_band_rows(int tile, int ntiles, int per_sm)
+{
+    for (int br = 16; br > (tile == 32 ? 4 : 8); br /= 2)
+        if ((int64_t)ntiles * (tile / br) >= per_sm * 152) return br;
+    return tile == 32 ? 4 : 8;
+}
+
 // FP64 tiles of a step without the monitor, in bands of br rows, one CTA each
 // (kob_band_rows), so that a grid of few tiles reaches every SM: the FP64 pipe
 // of one SM works 211000 cycles on a 32^2 reference-order tile with general
@@ -376,14 +386,20 @@ __global__ void __launch_bounds__(kob_threads<T, TIER>()) kob_step_kernel(StepAr
 // in the reference's order (12 tiles): 113 us a step as whole tiles with general
 // divisions, 15 in bands; 256^2: 181 and 58; 512^2: 367 and 134; 1024^2: 1275
 // and 473.
-template <int T, bool REF>
-__global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __grid_constant__ StepArgs a, int br)
+template <int T, bool REF, int NT>
+__global__ void __launch_bounds__(NT) kob_step_f64_band_kernel(const __grid_constant__ StepArgs a, int br)
 {
     constexpr int W = T + 4, E = T + 2;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ uint8_t ntier[9];
     pdl_wait();
     pdl_trigger();
+    if (br == 0) {
+        br = kob_band_rows(T, a.count[TIER_FP64], 2);
+        // one pass of the CTAs in place of one and a part
+        const int n = a.count[TIER_FP64] * (T / br);
+        if (br < 16 && n > (int)gridDim.x && n < 2 * (int)gridDim.x) br *= 2;
+    }
     const int nb = T / br, items = a.count[TIER_FP64] * nb;
     if ((int)blockIdx.x >= items) return;
     double *sp = reinterpret_cast<double *>(smraw), *st = sp + (br + 4) * W;  // phi, T
@@ -396,12 +412,12 @@ __global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __gri
         const int x0 = tx * T, y0 = ty * T;
         load_neighbour_tiers(a, tx, ty, ntier);
         __syncthreads();  // (also: the previous item's reads of the staging)
-        stage_band<T, 2>(a, sp, ntier, tx, ty, ly0 - 2, br + 4, 0, 2);
+        stage_band<T, 2, NT>(a, sp, ntier, tx, ty, ly0 - 2, br + 4, 0, 2);
         stage_band_wait();
         __syncthreads();
         // with zero flux an out-of-domain ring cell takes the values of the
         // cell it mirrors, which lies in the same band
-        for (int u = threadIdx.x; u < (br + 2) * E; u += kThreads) {
+        for (int u = threadIdx.x; u < (br + 2) * E; u += NT) {
             int ly = ly0 - 1 + u / E, lx = u % E - 1;
             if (a.bc != 0) {
                 lx = bc_map(x0 + lx, a.nx, 1) - x0;
@@ -410,7 +426,7 @@ __global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __gri
             kob_aniso64<REF>(sp + (ly - ly0 + 2) * W + lx + 2, W, ph, a1[u], a2[u], ep[u]);
         }
         __syncthreads();
-        for (int u = threadIdx.x; u < br * T; u += kThreads) {
+        for (int u = threadIdx.x; u < br * T; u += NT) {
             const int i = u % T, j = u / T;
             const int64_t g = (int64_t)(y0 + ly0 + j) * a.nx + x0 + i;
             const int c = (j + 2) * W + i + 2;
@@ -422,30 +438,38 @@ __global__ void __launch_bounds__(kThreads) kob_step_f64_band_kernel(const __gri
     }
 }
 
-// Rows of a band: the most that still give the grid's tiles four CTAs an SM
-// (a band recomputes phase A on two extra rows: 1.5, 1.25, 1.13 times the
-// tile's rows for bands of 4, 8 and 16).
-static int kob_band_rows(int tile, int ntiles)
-{
-    for (int br = 16; br > (tile == 32 ? 4 : 8); br /= 2)
-        if ((int64_t)ntiles * (tile / br) >= 4 * 152) return br;
-    return tile == 32 ? 4 : 8;
-}
-
 template <int T> static size_t kob_band_smem(int br)
 {
     return sizeof(double) * (2 * (size_t)(br + 4) * (T + 4) + 3 * (size_t)(br + 2) * (T + 2));
 }
 
-template <int T>
-static cudaError_t kob_launch_band(bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl)
+template <int T, int NT>
+static cudaError_t kob_launch_band(bool ref, const StepArgs &a, int br, int ctas, size_t smem, cudaStream_t s, bool pdl)
 {
-    // where other tiers are in use the FP64 tiles are few, often none: one CTA
-    // an SM, which loop over the bands
-    const bool mixed = a.in[TIER_HALF] != nullptr || a.in[TIER_FP32] != nullptr;
-    const int br = kob_band_rows(T, mixed ? 0 : grid), n = grid * (T / br), ctas = mixed && n > 152 ? 152 : n;
-    return ref ? launch_kernel(kob_step_f64_band_kernel<T, true>, ctas, kob_band_smem<T>(br), s, pdl, a, br)
-               : launch_kernel(kob_step_f64_band_kernel<T, false>, ctas, kob_band_smem<T>(br), s, pdl, a, br);
+    return ref ? launch_kernel_nt(kob_step_f64_band_kernel<T, true, NT>, ctas, NT, smem, s, pdl, a, br)
+               : launch_kernel_nt(kob_step_f64_band_kernel<T, false, NT>, ctas, NT, smem, s, pdl, a, br);
+}
+
+// Plain FP64 runs: a CTA a band.  Adaptive runs, whose FP64 tiles only the
+// device can count (br = 0): CTAs that loop over the bands, as many as tiles
+// but at least one and at most four an SM, since each also costs a step without
+// FP64 tiles its start; of 512 threads, so that an SM takes no more than four of
+// those that start while the previous step drains.  512^2, 16^2 tiles, a third
+// of them FP64, us a step: whole tiles 43 (reference order 86), a CTA of 256
+// threads an SM and 8-row bands 84 (97), this 40 (53); 32^2 tiles, 44% FP64: 68
+// (148), 100 (122), 66 (93).  few: no tile is expected at FP64: one small CTA an SM
+// (the tuned 512^2 run 7.6 us a step, against 7.8-8.4 with more or larger CTAs).
+template <int T>
+static cudaError_t kob_launch_bands(bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl, bool few)
+{
+    const bool plain = a.in[TIER_HALF] == nullptr && a.in[TIER_FP32] == nullptr;
+    if (plain || few) {
+        const int br = kob_band_rows(T, plain ? grid : 0, 4), n = grid * (T / br);
+        return kob_launch_band<T, kThreads>(ref, a, br, plain || n < 152 ? n : 152, kob_band_smem<T>(br), s, pdl);
+    }
+    const int n = grid * (T / kob_band_rows(T, 0, 2));  // bands at most
+    const int cap = grid < 152 ? 152 : (grid < 4 * 152 ? grid : 4 * 152);
+    return kob_launch_band<T, 512>(ref, a, 0, n < cap ? n : cap, kob_band_smem<T>(16), s, pdl);
 }
 
 // The half and FP32 tiles of a step in one launch (one CTA per tile; FP64
@@ -491,7 +515,7 @@ size_t kob_smem_bytes(int tile, int tier)
 static bool kob_poly(const StepArgs &a) { return a.ph.kf[KB_MODE] != 0.f; }
 
 template <int T>
-static cudaError_t kob_launch_tt(int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl)
+static cudaError_t kob_launch_tt(int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl, bool few)
 {
     const bool poly = kob_poly(a);
     switch (tier) {
@@ -502,15 +526,16 @@ static cudaError_t kob_launch_tt(int tier, bool ref, const StepArgs &a, int grid
         return poly ? kob_launch_t<T, TIER_FP32, false, true>(a, grid, s, pdl)
                     : kob_launch_t<T, TIER_FP32, false, false>(a, grid, s, pdl);
     default:
-        if (!a.monitor_now) return kob_launch_band<T>(ref, a, grid, s, pdl);
+        if (!a.monitor_now) return kob_launch_bands<T>(ref, a, grid, s, pdl, few);
         return ref ? kob_launch_t<T, TIER_FP64, true, false>(a, grid, s, pdl)
                    : kob_launch_t<T, TIER_FP64, false, false>(a, grid, s, pdl);
     }
 }
 
-cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl)
+cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid, cudaStream_t s, bool pdl, bool few)
 {
-    return tile == 32 ? kob_launch_tt<32>(tier, ref, a, grid, s, pdl) : kob_launch_tt<16>(tier, ref, a, grid, s, pdl);
+    return tile == 32 ? kob_launch_tt<32>(tier, ref, a, grid, s, pdl, few)
+                      : kob_launch_tt<16>(tier, ref, a, grid, s, pdl, few);
 }
 
 // the monitor steps take the variant with the monitor compiled in, runs
