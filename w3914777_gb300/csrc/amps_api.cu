@@ -1433,7 +1433,7 @@ extern "C" int amps_ensemble_create(amps_handle *const *members, int count, amps
     e->mixed = h0->mixed;
     e->ref = h0->p.ref_order != 0;
     // groups: members with the larger staging first, whose size a group's launches
-    // take (16^2 tiles: 16 fields stage more than 17, gg_fp64_band); a group closes
+    // take (16^2 tiles: 12 fields stage more than 13, gg_fp64_band); a group closes
     // where the occupancy that its first member's staging allows would change, or at kEnsCap
     auto staging = [&](int i) { return gg_ens_smem_bytes(e->T, members[i]->nf); };
     std::vector<int> order(count);

@@ -13,7 +13,8 @@ cudaError_t kob_launch(int tile, int tier, bool ref, const StepArgs &a, int grid
                        bool few = false);
 cudaError_t sint_launch(int tile, int tier, bool ref, bool mu64, const StepArgs &a, int grid, cudaStream_t s,
                         bool pdl = false);
-size_t gg_smem_bytes(int tile, int nf);
+// f64: FP64 tiles are in use
+size_t gg_smem_bytes(int tile, int nf, bool f64 = true);
 // Kobayashi / sintering: the half and FP32 tiles of a step in one launch
 // (grid = all tiles; FP64 tiles are skipped, left to the FP64 tier launch).
 // after64: this step's FP64 launch directly precedes (run alongside it)

@@ -258,8 +258,9 @@ template <int T> struct Stage64 {
 
 // Rows of a band of `nf` fields: the most that fit in the FP32 staging of a
 // 32^2 tile (16 rows of 36 doubles against 34 of 40 floats, and the sum tile
-// in that of the sums of squares); a 16^2 tile whole, up to 16 fields.
-__host__ __device__ __forceinline__ int gg_fp64_band(int tile, int nf) { return tile == 32 ? 16 : (nf <= 16 ? 16 : 8); }
+// in that of the sums of squares); a 16^2 tile whole, up to 12 fields (with 16 an
+// SM's four CTAs would take 196 KB: steps without FP64 tiles 2% slower).
+__host__ __device__ __forceinline__ int gg_fp64_band(int tile, int nf) { return tile == 32 ? 16 : (nf <= 12 ? 16 : 8); }
 
 // Stage rows [r0 - 1, r0 + hb] of every field (tile-local), each cell read at
 // its owner tile's input tier: the tile of the 3x3 neighbourhood at that
@@ -269,11 +270,11 @@ __host__ __device__ __forceinline__ int gg_fp64_band(int tile, int nf) { return 
 // ALL64: every cell is at FP64 (no tier is looked up).
 template <int T, bool NC, bool ALL64 = false>
 __device__ __forceinline__ void gg_stage64(const StepArgs &a, double *sm, const uint8_t *nt, int x0, int y0, int r0,
-                                           int hb, bool own)
+                                           int hb, bool own, int tid)
 {
     using S = Stage64<T>;
     const int nf = a.nf, fs = S::field(hb);
-    for (int u = threadIdx.x; u < (hb + 2) * (T + 2); u += kThreads) {
+    for (int u = tid; u < (hb + 2) * (T + 2); u += kThreads) {
         const int ly = r0 - 1 + u / (T + 2), lx = u % (T + 2) - 1;
         const int gy = bc_map(y0 + ly, a.ny, a.bc), gx = bc_map(x0 + lx, a.nx, a.bc);
         const int cls = (ly < 0 ? 0 : (ly < T ? 3 : 6)) + (lx < 0 ? 0 : (lx < T ? 1 : 2));
@@ -303,7 +304,7 @@ __device__ __forceinline__ void gg_stage64(const StepArgs &a, double *sm, const 
 // The monitor of an FP64 tile, from the values just stored (exact) and the
 // tile's input: one pass over the tile after the update, on monitor steps only.
 template <int T, int KIND>
-__device__ __forceinline__ void gg_monitor64(const StepArgs &a, const uint8_t *nt, int tile, int tx, int ty, double *red)
+__device__ __forceinline__ void gg_monitor64(const StepArgs &a, const uint8_t *nt, int tile, int tx, int ty, double *red, int tid)
 {
     const int x0 = tx * T, y0 = ty * T;
     // a ragged grid's edge tile: cells past the domain are not samples
@@ -316,7 +317,7 @@ __device__ __forceinline__ void gg_monitor64(const StepArgs &a, const uint8_t *n
         if (a.mfield >= 0 && a.mfield != f) continue;
         const int mslot = a.mfield < 0 ? f : 0;
         if (range) mon_reset(a, mon);
-        for (int u = threadIdx.x; u < T * T; u += kThreads) {
+        for (int u = tid; u < T * T; u += kThreads) {
             const int row = u / T, col = u % T;
             if (row >= vh || col >= vw) continue;
             const int64_t g = (int64_t)(y0 + row) * a.px + x0 + col, k = (int64_t)f * a.n + g;
@@ -332,14 +333,15 @@ __device__ __forceinline__ void gg_monitor64(const StepArgs &a, const uint8_t *n
         if (range) metric = mon_finish(a, mon, red, metric);
     }
     if (!range) metric = mon_finish(a, mon, red, metric);
-    if (threadIdx.x == 0) a.metric[tile] = metric;
+    if (tid == 0) a.metric[tile] = metric;
 }
 
-// The update of one band from its staging (rows [r0, r0 + hb) of the tile),
-// fields [f0, f0 + fn) (the sums cover every field).
+// The update of every field in one band (rows [r0, r0 + hb) of the tile) from
+// its staging; a lane takes RR rows x 2 columns.  rot: added to a warp's index
+// where it picks its fields.
 template <int T, bool REF, int RR>
 __device__ __forceinline__ void gg_band64(const StepArgs &a, const double *sm, double *ss, int x0, int y0, int r0,
-                                          int hb, int rot)
+                                          int hb, int rot, int tid)
 {
     using S = Stage64<T>;
     constexpr int GPR = T / 2, RG = 32 / GPR;  // column pairs a row, row groups a warp
@@ -347,7 +349,7 @@ __device__ __forceinline__ void gg_band64(const StepArgs &a, const double *sm, d
     const Phys &ph = a.ph;
     if (!REF) {
         // G = 2 gamma S - 1 at every cell of the band
-        for (int u = threadIdx.x; u < hb * GPR; u += kThreads) {
+        for (int u = tid; u < hb * GPR; u += kThreads) {
             const int row = u / GPR, c = 2 * (u % GPR);
             const double *p = sm + (row + 1) * S::P + S::O + c;
             double s0 = 0.0, s1 = 0.0;
@@ -361,7 +363,7 @@ __device__ __forceinline__ void gg_band64(const StepArgs &a, const double *sm, d
         }
         __syncthreads();
     }
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) + rot;
+    const int lane = tid & 31, warp = (tid >> 5) + rot;
     const int c = 2 * (lane % GPR);
     const int parts = hb / (RG * RR);  // warps that share a field
     for (int u = warp & 7; u < nf * parts; u += kThreads / 32) {
@@ -473,45 +475,63 @@ __device__ __forceinline__ void gg_band64(const StepArgs &a, const double *sm, d
 
 // Rows [row0, row1) of an FP64 tile in bands of hb rows (the whole tile but
 // for a CTA of a split tile), by the whole CTA, in the CTA's staging memory
-// (no copy into it may be in flight).  Out of line: the FP32 path's registers
-// are not shared with it.
+// (no copy into it may be in flight).
 template <int T, bool REF, bool NC = true>
 __device__ __forceinline__ void gg_tile_fp64(const StepArgs &a, float *smf, const uint8_t *nt, int tile, int tx, int ty,
-                                          double *red, int row0, int row1, int hb)
+                                          double *red, int row0, int row1, int hb, int tid)
 {
     double *sm = reinterpret_cast<double *>(smf);
     double *ss = sm + a.nf * Stage64<T>::field(hb);
     const int x0 = tx * T, y0 = ty * T;
     const bool own = (tx + 1) * T > a.nx || (ty + 1) * T > a.ny;  // a ragged grid's edge tile
     for (int r0 = row0; r0 < row1; r0 += hb) {
-        gg_stage64<T, NC>(a, sm, nt, x0, y0, r0, hb, own);
+        gg_stage64<T, NC>(a, sm, nt, x0, y0, r0, hb, own, tid);
         __syncthreads();
         // the warps' fields rotate with the tile, so that CTAs with fewer
         // fields than warps load every SM sub-partition's FP64 pipe
         const int rot = 2 * (tile & 3);
-        if (T == 32 && hb == 16 && a.nf % 8 == 0) gg_band64<T, REF, T == 32 ? 8 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
-        else if (T == 32 && hb == 16) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        if (T == 32 && hb == 16 && a.nf % 8 == 0) gg_band64<T, REF, T == 32 ? 8 : 2>(a, sm, ss, x0, y0, r0, hb, rot, tid);
+        else if (T == 32 && hb == 16) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot, tid);
         // (one row a lane keeps all eight warps of a two-field 16^2 tile busy:
         // 32.4 -> 30.1 us a step of the reference's 512^2 adaptive run)
-        else if (REF && a.nf <= 2) gg_band64<T, REF, REF ? 1 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
-        else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot);
+        else if (REF && a.nf <= 2) gg_band64<T, REF, REF ? 1 : 2>(a, sm, ss, x0, y0, r0, hb, rot, tid);
+        else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot, tid);
         __syncthreads();  // the next band overwrites the staging; the monitor reads the stored tile
     }
     if (a.monitor_now) {
-        if (a.monitor_kind == 3) gg_monitor64<T, 3>(a, nt, tile, tx, ty, red);
-        else if (a.monitor_kind == 2) gg_monitor64<T, 2>(a, nt, tile, tx, ty, red);
-        else gg_monitor64<T, 1>(a, nt, tile, tx, ty, red);
+        if (a.monitor_kind == 3) gg_monitor64<T, 3>(a, nt, tile, tx, ty, red, tid);
+        else if (a.monitor_kind == 2) gg_monitor64<T, 2>(a, nt, tile, tx, ty, red, tid);
+        else gg_monitor64<T, 1>(a, nt, tile, tx, ty, red, tid);
     }
 }
 
-// The same out of line, for the ensemble's kernels (and ragged steps without a
-// monitor): inlined there, its registers pushed the FP32 path into spills (64
-// members, 1000 steady FP32 steps: 305 ms inlined, 298 out of line).
+// The speculative staging copies have landed (false: a bounded wait on the
+// tensor copy gave up -- flagged; the CTA waits once more for it and returns).
+__device__ __forceinline__ bool gg_copies_landed(const StepArgs &a, bool bulk, uint64_t *bar)
+{
+    if (!bulk) {
+        cp_async_wait_all();
+        return true;
+    }
+    const bool ok = mbar_wait_bounded(bar, 0);
+    if (__syncthreads_or(!ok)) {
+        if (threadIdx.x == 0) {
+            atomicOr(a.flags, 2);
+            if (!ok) mbar_wait_bounded(bar, 0);
+        }
+        return false;
+    }
+    return true;
+}
+
+// The same out of line, after the discarded copies (see gg_tile_step).
 template <int T, bool REF, bool NC = true>
 __device__ __noinline__ void gg_tile_fp64_call(const StepArgs &a, float *smf, const uint8_t *nt, int tile, int tx, int ty,
-                                               double *red)
+                                               double *red, bool spec, bool bulk, uint64_t *bar)
 {
-    gg_tile_fp64<T, REF, NC>(a, smf, nt, tile, tx, ty, red, 0, T, gg_fp64_band(T, a.nf));
+    if (spec && !gg_copies_landed(a, bulk, bar)) return;
+    if (spec && !bulk) __syncthreads();  // every thread's own copies
+    gg_tile_fp64<T, REF, NC>(a, smf, nt, tile, tx, ty, red, 0, T, gg_fp64_band(T, a.nf), (int)threadIdx.x);
 }
 
 __device__ __forceinline__ __half2 gg_hconst(const Phys &ph, int i)
@@ -682,15 +702,26 @@ __device__ __forceinline__ bool all_fp32(const uint8_t *nt)
 // reads values that other CTAs of the same launch wrote).  RG: the grid may
 // be ragged (its edge tiles partial); compiled out of the whole-tile grids'
 // kernels, whose registers it would otherwise spill.
+// F64 = false: no tile of the run is ever at FP64 (and REF says nothing).
+// How the FP64 path is kept off the other tiles' way: out of line (the
+// ensemble, ragged steps without a monitor, 16^2 tiles), or, in the reference's
+// order, where a call costs 8-15% of an all-FP64 step, behind opaque copies of
+// what its addresses and indices come from, which the compiler otherwise
+// forms ahead of the branch.  512^2, 16^2 tiles, us a step without / with
+// all tiles at FP64: plainly inlined 7.80 / 29.3, called 7.19 / 32.9, opaque
+// 7.45 / 29.2; the library's order, half tiles of 8 fields: 11.35 inlined, 11.15
+// called.  (32^2 tiles in the library's order: 13.9 us a 1024^2 step inlined
+// plainly, 14.1 with opaque copies, up to 4% more called.)
 // tm, bar (T = 32): a tensor map of this step's FP32 input and an mbarrier;
 // tiles whose halo needs no wrap or mirror then fetch the whole FP32
 // neighbourhood -- every field, 34 rows x 40 columns, the staging layout --
 // by one bulk tensor copy issued by one thread (sm 128-byte aligned).
-template <int T, bool REF, int MK, int HA = 0, bool NC = true, bool RG = false>
+template <int T, bool REF, int MK, int HA = 0, bool NC = true, bool RG = false, bool F64 = true>
 __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8_t *ntier, double *red, int tile,
                                              const CUtensorMap *tm = nullptr, uint64_t *bar = nullptr)
 {
     constexpr bool MON = MK != 0;
+    constexpr bool kFp64Call = (T == 16 && !REF) || (RG && MK <= 0);
     const int tx = tile % a.ntx, ty = tile / a.ntx;
     load_neighbour_tiers(a, tx, ty, ntier);
     // the copy of the FP32 neighbourhood (the common case) starts before the
@@ -698,7 +729,7 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
     // turns out FP64 or its neighbourhood mixed, the copies are drained and
     // their data (in-bounds reads of the full-size FP32 store) discarded
     // (not when every tile is known to be FP64)
-    const bool spec = T == 32 && a.in[TIER_FP32] != nullptr && !a.all64;
+    const bool spec = T == 32 && a.in[TIER_FP32] != nullptr && !(F64 && a.all64);
     const bool bulk = spec && tm != nullptr && tx >= 1 && ty >= 1 && tx <= a.ntx - 2 && ty <= a.nty - 2;
     if (bulk) {
         if (threadIdx.x == 0) {
@@ -710,31 +741,20 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
     } else if (spec) {
         stage_tile_async32<T, 1, false>(a, sm, tx, ty, a.nf);
     }
-    // the staging copies have landed (false: a bounded wait on the tensor
-    // copy gave up -- flagged; the CTA waits once more for it and returns)
-    auto spec_done = [&]() -> bool {
-        if (!bulk) {
-            cp_async_wait_all();
-            return true;
-        }
-        const bool ok = mbar_wait_bounded(bar, 0);
-        if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0) {
-                atomicOr(a.flags, 2);
-                if (!ok) mbar_wait_bounded(bar, 0);
-            }
-            return false;
-        }
-        return true;
-    };
+    auto spec_done = [&]() -> bool { return gg_copies_landed(a, bulk, bar); };
     const int tier = a.tier_out[tile];
     __syncthreads();
-    if (tier == TIER_FP64) {
+    if (F64 && tier == TIER_FP64) {
         // the FP64 bands are staged in the same memory: the discarded copies land first
-        if (spec && !spec_done()) return;
-        if (spec && !bulk) __syncthreads();  // every thread's own copies
-        if constexpr (RG && MK <= 0) gg_tile_fp64_call<T, REF, NC>(a, sm, ntier, tile, tx, ty, red);
-        else gg_tile_fp64<T, REF, NC>(a, sm, ntier, tile, tx, ty, red, 0, T, gg_fp64_band(T, a.nf));
+        if constexpr (kFp64Call) {
+            gg_tile_fp64_call<T, REF, NC>(a, sm, ntier, tile, tx, ty, red, spec, bulk, bar);
+        } else {
+            int tid = (int)threadIdx.x, x = tx, y = ty;
+            if constexpr (REF) asm volatile("" : "+r"(tid), "+r"(tile), "+r"(x), "+r"(y), "+l"(sm)::"memory");
+            if (spec && !spec_done()) return;
+            if (spec && !bulk) __syncthreads();  // every thread's own copies
+            gg_tile_fp64<T, REF, NC>(a, sm, ntier, tile, x, y, red, 0, T, gg_fp64_band(T, a.nf), tid);
+        }
         return;
     }
     const bool all32 = all_fp32(ntier);
@@ -800,7 +820,7 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
 // their neighbourhood in shared memory (reading it directly through L1
 // measured 18.1 against 15.8 us per adaptive 1024^2 Q=8 step).
 // tm: the tensor map of the step's FP32 input, valid when a.tma_stage.
-template <int T, bool REF, int MK, int HA = 0, bool RG = false>
+template <int T, bool REF, int MK, int HA = 0, bool RG = false, bool F64 = true>
 __global__ void __launch_bounds__(kThreads, 4) gg_step_kernel(const __grid_constant__ StepArgs a, const __grid_constant__ CUtensorMap tm)
 {
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -816,7 +836,7 @@ __global__ void __launch_bounds__(kThreads, 4) gg_step_kernel(const __grid_const
     pdl_trigger();
     pdl_wait();
     const int tile = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
-    gg_tile_step<T, REF, MK, HA, true, RG>(a, sm, ntier, red, tile, a.tma_stage ? &tm : nullptr, &bar);
+    gg_tile_step<T, REF, MK, HA, true, RG, F64>(a, sm, ntier, red, tile, a.tma_stage ? &tm : nullptr, &bar);
 }
 
 

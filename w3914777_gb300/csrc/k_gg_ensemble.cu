@@ -92,7 +92,8 @@ __device__ __forceinline__ void gg_tile_pair(const StepArgs &a, float *sm, uint8
         // field, and the staging memory is that of half of them)
         if (spec && !spec_done()) return;
         __syncthreads();
-        gg_tile_fp64<T, REF>(a, sm, ntier, tile, tx, ty, red, (int)rank * 16, (int)rank * 16 + 16, 4);
+        gg_tile_fp64<T, REF>(a, sm, ntier, tile, tx, ty, red, (int)rank * 16, (int)rank * 16 + 16, 4,
+                             (int)threadIdx.x);
         return;
     }
     const bool all32 = all_fp32(ntier);

@@ -29,6 +29,14 @@ static cudaError_t launch_ref(bool ref, const StepArgs &a, int grid, size_t smem
 cudaError_t gg_launch_half(int tile, bool ref, const StepArgs &a, int grid, size_t smem, cudaStream_t s,
                            const CUtensorMap &tm)
 {
+    if (a.in[TIER_FP64] == nullptr && !a.monitor_now) {  // a half run: no FP64 code
+        if (a.half_arith == 1)
+            return tile == 32 ? launch_kernel(gg_step_kernel<32, false, 0, 1, false, false>, grid, smem, s, true, a, tm)
+                              : launch_kernel(gg_step_kernel<16, false, 0, 1, false, false>, grid, smem, s, true, a, tm);
+        if (a.half_arith == 2)
+            return tile == 32 ? launch_kernel(gg_step_kernel<32, false, 0, 2, false, false>, grid, smem, s, true, a, tm)
+                              : launch_kernel(gg_step_kernel<16, false, 0, 2, false, false>, grid, smem, s, true, a, tm);
+    }
     if (a.half_arith == 1)
         return tile == 32 ? launch_ref<32, 1>(ref, a, grid, smem, s, tm) : launch_ref<16, 1>(ref, a, grid, smem, s, tm);
     if (a.half_arith == 2)
@@ -41,7 +49,8 @@ static cudaError_t prepare_mk()
 {
     const int lim = kMaxDynSmem;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 0, HA>, attr, lim);
+    cudaError_t e = cudaFuncSetAttribute(gg_step_kernel<T, false, 0, HA, false, false>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 0, HA>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 1, HA>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 2, HA>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 3, HA>, attr, lim);

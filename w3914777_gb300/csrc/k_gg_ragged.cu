@@ -24,6 +24,9 @@ static cudaError_t launch_mk(const StepArgs &a, int grid, size_t smem, cudaStrea
 cudaError_t gg_launch_ragged(int tile, bool ref, const StepArgs &a, int grid, size_t smem, cudaStream_t s,
                              const CUtensorMap &tm)
 {
+    if (a.in[TIER_FP64] == nullptr && !a.monitor_now)  // a half or FP32 run: no FP64 code
+        return tile == 32 ? launch_kernel(gg_step_kernel<32, false, 0, 0, true, false>, grid, smem, s, true, a, tm)
+                          : launch_kernel(gg_step_kernel<16, false, 0, 0, true, false>, grid, smem, s, true, a, tm);
     if (tile == 32) return ref ? launch_mk<32, true>(a, grid, smem, s, tm) : launch_mk<32, false>(a, grid, smem, s, tm);
     return ref ? launch_mk<16, true>(a, grid, smem, s, tm) : launch_mk<16, false>(a, grid, smem, s, tm);
 }
@@ -33,7 +36,8 @@ static cudaError_t prepare_mk()
 {
     const int lim = kMaxDynSmem;
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 0, 0, true>, attr, lim);
+    cudaError_t e = cudaFuncSetAttribute(gg_step_kernel<T, false, 0, 0, true, false>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 0, 0, true>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 1, 0, true>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 2, 0, true>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gg_step_kernel<T, REF, 3, 0, true>, attr, lim);

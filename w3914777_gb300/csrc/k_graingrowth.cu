@@ -22,7 +22,7 @@
 namespace amps {
 
 // A step whose tiles are all read and written at FP64 (plain FP64 runs, and an
-// adaptive run's first period): a CTA per band of hb rows of a tile, so that
+// adaptive run's first period): a CTA per band of hb = 8 rows of a tile, so that
 // the FP64 pipes of all SMs fill evenly.  No tiers and no monitor (monitor
 // steps take the fused kernel).  FP64-pipe bound.  A plain 512^2 Q=8 step (256
 // tiles): 77 us with whole tiles and 18 operations a cell and field, 48 with
@@ -37,11 +37,11 @@ __global__ void __launch_bounds__(kThreads, 4) gg_step_f64_kernel(const __grid_c
     pdl_wait();
     const int nb = T / hb, tile = blockIdx.x / nb, r0 = (int)(blockIdx.x % nb) * hb;
     const int x0 = tile % a.ntx * T, y0 = tile / a.ntx * T;
-    gg_stage64<T, true, true>(a, sm, nullptr, x0, y0, r0, hb, false);
+    gg_stage64<T, true, true>(a, sm, nullptr, x0, y0, r0, hb, false, (int)threadIdx.x);
     __syncthreads();
     const int rot = 2 * ((int)blockIdx.x & 3);  // as in gg_tile_fp64
-    if (T == 32 && a.nf >= 8) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot);
-    else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot);
+    if (T == 32 && a.nf >= 8) gg_band64<T, REF, T == 32 ? 4 : 2>(a, sm, ss, x0, y0, r0, hb, rot, (int)threadIdx.x);
+    else gg_band64<T, REF, 2>(a, sm, ss, x0, y0, r0, hb, rot, (int)threadIdx.x);
 }
 
 // ---- multi-step kernel ---------------------------------------------------------
@@ -145,7 +145,7 @@ cudaError_t gg_launch_flow(bool ref, const StepArgs &a0, const StepArgs &a1, con
     return cudaGetLastError();
 }
 
-size_t gg_smem_bytes(int tile, int nf)
+size_t gg_smem_bytes(int tile, int nf, bool f64)
 {
     // 32^2: + the sum-of-squares tile of gg_tile_lo_rows; + 128 bytes to align
     // the staging for tensor copies (gg_step_kernel).  FP64 tiles use the same
@@ -153,7 +153,7 @@ size_t gg_smem_bytes(int tile, int nf)
     if (tile == 32) return ((size_t)nf * Stage<float, 32, 1>::FIELD + 32 * 32) * sizeof(float) + 128;
     const int hb = gg_fp64_band(16, nf);
     const size_t lo = (size_t)nf * Stage<float, 16, 1>::FIELD * sizeof(float);
-    const size_t hi = ((size_t)nf * Stage64<16>::field(hb) + hb * 16) * sizeof(double);
+    const size_t hi = f64 ? ((size_t)nf * Stage64<16>::field(hb) + hb * 16) * sizeof(double) : 0;
     return (lo > hi ? lo : hi) + 128;
 }
 
@@ -180,7 +180,8 @@ cudaError_t gg_launch(int tile, bool ref, const StepArgs &a, int grid, cudaStrea
         return ref ? launch_kernel(gg_step_f64_kernel<16, true>, n, sm64, s, true, a, hb)
                    : launch_kernel(gg_step_f64_kernel<16, false>, n, sm64, s, true, a, hb);
     }
-    const size_t smem = gg_smem_bytes(tile, a.nf);
+    const bool f64 = a.in[TIER_FP64] != nullptr;
+    const size_t smem = gg_smem_bytes(tile, a.nf, f64);
 #define AMPS_GGK(TT, MK)                                                                              \
     do {                                                                                              \
         if (ref) return launch_pdl(gg_step_kernel<TT, true, MK>, grid, smem, s, a, tm);               \
@@ -199,6 +200,9 @@ cudaError_t gg_launch(int tile, bool ref, const StepArgs &a, int grid, cudaStrea
         return gg_launch_ragged(tile, ref, a, grid, smem, s, tm);  // partial edge tiles (k_gg_ragged.cu)
     } else if (a.half_arith != 0) {
         return gg_launch_half(tile, ref, a, grid, smem, s, tm);  // binary16 half tiles (k_gg_half.cu)
+    } else if (!f64 && !a.monitor_now) {  // a half or FP32 run: no FP64 code
+        return tile == 32 ? launch_pdl(gg_step_kernel<32, false, 0, 0, false, false>, grid, smem, s, a, tm)
+                          : launch_pdl(gg_step_kernel<16, false, 0, 0, false, false>, grid, smem, s, a, tm);
     } else {
         if (tile == 32) AMPS_GGM(32);
         else AMPS_GGM(16);
@@ -219,6 +223,8 @@ cudaError_t gg_prepare(int tile, bool ref, int half_arith, bool ragged)
     if (e != cudaSuccess) return e;
     if (half_arith != 0) return gg_prepare_half(tile, ref, half_arith);
     if (ragged) return gg_prepare_ragged(tile, ref);
+    e = tile == 32 ? cudaFuncSetAttribute(gg_step_kernel<32, false, 0, 0, false, false>, attr, lim)
+                   : cudaFuncSetAttribute(gg_step_kernel<16, false, 0, 0, false, false>, attr, lim);
 #define AMPS_GGP(TT, MK)                                                                                     \
     if (e == cudaSuccess)                                                                                    \
         e = ref ? cudaFuncSetAttribute(gg_step_kernel<TT, true, MK>, attr, lim)                              \
@@ -320,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             load_neighbour_tiers(a, tx, ty, ntier);
             __syncthreads();
             if (tier == TIER_FP64) {
-                gg_tile_fp64<T, REF>(a, sm, ntier, t, tx, ty, red, 0, T, gg_fp64_band(T, a.nf));
+                gg_tile_fp64<T, REF>(a, sm, ntier, t, tx, ty, red, 0, T, gg_fp64_band(T, a.nf), (int)threadIdx.x);
             } else {
                 stage_tile<float, T, 1>(a, sm, ntier, tx, ty, 0, a.nf);
                 __syncthreads();
