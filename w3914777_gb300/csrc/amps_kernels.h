@@ -61,7 +61,7 @@ cudaError_t gg_launch_tma(bool ref, const CUtensorMap &tm, const StepArgs &a, in
 // Ensemble step: one launch per group of members, one CTA per (member, tile)
 // work item; the group's step arguments travel by value in the kernel's
 // parameter space (up to kEnsCap members), read through the constant cache.
-constexpr int kEnsCap = 40;
+constexpr int kEnsCap = 38;
 struct EnsLaunch {
     int count;               // members in this launch
     int first[kEnsCap + 1];  // first CTA of each member; first[count] = the grid

@@ -712,11 +712,16 @@ __device__ __forceinline__ bool all_fp32(const uint8_t *nt)
 // 7.45 / 29.2; the library's order, half tiles of 8 fields: 11.35 inlined, 11.15
 // called.  (32^2 tiles in the library's order: 13.9 us a 1024^2 step inlined
 // plainly, 14.1 with opaque copies, up to 4% more called.)
+// TT: the thread that issues the tensor copy.  The ensemble's launches take one
+// that loads no neighbour's tier: thread 0 waits for its tier first (1000 steady
+// steps of 64 members: 298 ms with thread 0, 292 with thread 32; a single run's
+// small grids are faster with thread 0).
 // tm, bar (T = 32): a tensor map of this step's FP32 input and an mbarrier;
 // tiles whose halo needs no wrap or mirror then fetch the whole FP32
 // neighbourhood -- every field, 34 rows x 40 columns, the staging layout --
 // by one bulk tensor copy issued by one thread (sm 128-byte aligned).
-template <int T, bool REF, int MK, int HA = 0, bool NC = true, bool RG = false, bool F64 = true>
+template <int T, bool REF, int MK, int HA = 0, bool NC = true, bool RG = false, bool F64 = true,
+          int TT = 0>
 __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8_t *ntier, double *red, int tile,
                                              const CUtensorMap *tm = nullptr, uint64_t *bar = nullptr)
 {
@@ -732,7 +737,7 @@ __device__ __forceinline__ void gg_tile_step(const StepArgs &a, float *sm, uint8
     const bool spec = T == 32 && a.in[TIER_FP32] != nullptr && !(F64 && a.all64);
     const bool bulk = spec && tm != nullptr && tx >= 1 && ty >= 1 && tx <= a.ntx - 2 && ty <= a.nty - 2;
     if (bulk) {
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == TT) {
             mbar_init(bar, 1);
             fence_mbar_init();
             mbar_arrive_expect_tx(bar, (uint32_t)(Stage<float, T, 1>::FIELD * a.nf * sizeof(float)));

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(kThreads, 4) gg_ens_kernel(const __grid_consta
         else hi = mid - 1;
     }
     const StepArgs &a = L.m[lo];
-    gg_tile_step<T, REF, MON ? -1 : 0, 0, true, true>(a, sm, ntier, red, b - L.first[lo], a.tmap, &bar);
+    gg_tile_step<T, REF, MON ? -1 : 0, 0, true, true, true, 32>(a, sm, ntier, red, b - L.first[lo], a.tmap, &bar);
 }
 
 // ---- split tiles ---------------------------------------------------------------
