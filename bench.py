@@ -514,8 +514,8 @@ def run_reference_cuda(steps=2000):
             "graingrowth", 1, mode="end2end_mix", monitor=m, monitor_samples=0, monitor_field=1, thr_lo=thr,
             thr_hi=thr, ref_order=1, half_arith=amps.HALF_REF, ref_snapshot=1))
         # the same run in the library's own arithmetic (FMA-form FP64 tiles,
-        # float arithmetic on half tiles): the reference order keeps
-        # pow(eta, 3) on the FP64 pipe, which paces the adaptive step
+        # float arithmetic on half tiles): the reference order takes its FP64
+        # tiles 2.6 times the FP64 operations
         gg[f"ours_mixed_fma_monitor{m}_{thr:g}"] = ours(amps.Params.preset(
             "graingrowth", 1, mode="end2end_mix", monitor=m, monitor_samples=0, monitor_field=1, thr_lo=thr,
             thr_hi=thr, ref_order=0))
